@@ -59,28 +59,6 @@ struct BatchDev {
     const CUtensorMap* maps;    // FP32: tensor map of buffer k's grid g at maps[k * ngrids + g] (null: per-field copies)
 };
 
-// dt of one step from the last CFL reduction (Solvers/EulerSolvers.cpp:130-161); the solver loop's
-// `while (t < t_final)` becomes `active`.
-CG_D void step_ctl_advance(StepCtl* c) {
-    if (!(c->t < c->t_final) || c->it >= c->it_limit) {
-        c->active = 0;
-        c->dt = 0.0;
-        return;
-    }
-    const double smax = __longlong_as_double((long long)c->smax[c->it & 1]);
-    double dt = c->cfl * (c->dx / smax);
-    if (c->it <= 5) dt = dt * 0.2;
-    if ((c->t + dt) > c->t_final) dt = c->t_final - c->t;
-    if (!(dt > 0.0) || !isfinite(dt)) c->status |= ST_NONFINITE;
-    c->dt = dt;
-    c->fc[0] = make_fast_coef(dt, c->dx);
-    c->fc[1] = make_fast_coef(dt * 0.5, c->dx);
-    c->active = 1;
-    c->smax[(c->it + 1) & 1] = 0ull;
-    c->t = c->t + dt;
-    c->it = c->it + 1;
-}
-
 // Grid-wide barrier for a cooperative launch.  Waits are bounded (b->limit polls of about 64 ns,
 // by default 2^26, about 4 s); a block that gives up sets err, and every block returns at its next
 // barrier (a block that is last to arrive passes, sees err and returns too).

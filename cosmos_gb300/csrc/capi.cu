@@ -463,8 +463,7 @@ int cosmos_grid_sweep(cosmos_grid* g, int axis, int order, double dt, double bia
     a.order = order;
     a.bias = bias;
     a.lim = limiter;
-    a.ds.fixed = dt;
-    a.ds.ffix = make_fast_coef(dt, g->p.dx);
+    a.ds.set_fixed(dt, g->p.dx);
     a.src = g->buf[g->cur];
     a.dst = g->buf[g->cur ^ 1];
     a.out.status = g->status;
@@ -481,7 +480,7 @@ int cosmos_grid_rk_source(cosmos_grid* g, double dt, double bias, int limiter) {
     SweepArgs a = base_args(g);
     a.bias = bias;
     a.lim = limiter;
-    a.ds.fixed = dt;
+    a.ds.set_fixed(dt, g->p.dx);
     a.src = g->buf[g->cur];
     a.dst = g->buf[g->cur ^ 1];
     a.out.status = g->status;

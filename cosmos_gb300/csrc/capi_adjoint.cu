@@ -271,15 +271,14 @@ extern "C" int cosmos_grid_adjoint(cosmos_grid* g, const cosmos_solve_opts* o, i
                 SweepArgs r = fa;
                 r.bias = 0.0;
                 r.lim = 1;
-                r.ds.fixed = dt;
+                r.ds.set_fixed(dt, g->p.dx);
                 r.src = slot(c, q);
                 r.dst = slot(c, q + 1);
                 ACK(launch_rk_source_exact(r));
                 continue;
             }
             fa.G.axis = axis;
-            fa.ds.fixed = dt;
-            fa.ds.ffix = make_fast_coef(dt, g->p.dx);
+            fa.ds.set_fixed(dt, g->p.dx);
             fa.src = slot(c, q);
             fa.dst = slot(c, q + 1);
             ACK(sweep_launch(g, fa));

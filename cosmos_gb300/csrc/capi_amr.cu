@@ -54,8 +54,7 @@ int masked_sweep(cosmos_grid* g, int axis, int order, double dt, const unsigned 
     a.order = order;
     a.bias = 0.0;
     a.lim = 1;
-    a.ds.fixed = dt;
-    a.ds.ffix = make_fast_coef(dt, g->p.dx);
+    a.ds.set_fixed(dt, g->p.dx);
     a.src = g->buf[g->cur];
     a.dst = g->buf[g->cur ^ 1];
     a.out.status = g->status;

@@ -3,6 +3,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "exact_math.cuh"
+
 namespace cg {
 
 #define CG_HD __host__ __device__ __forceinline__
@@ -49,6 +51,10 @@ CG_HD FastCoef make_fast_coef(double dt, double dx) {
     return FastCoef{(float)(dt / dx), (float)(0.5 * (dt / dx)), (float)(0.25 * (dx / dt))};
 }
 
+// dt / dx and dx / dt of a sweep (FP64)
+struct StepRatio { double d, c; };
+CG_HD StepRatio make_ratio(double dt, double dx) { return StepRatio{dt / dx, dx / dt}; }
+
 // Device-resident step controller.  The time step is computed on the device from the last
 // wavespeed reduction so that whole runs replay from a captured CUDA graph with no host sync.
 struct StepCtl {
@@ -63,6 +69,7 @@ struct StepCtl {
     int status;        // sticky error bits, see COSMOS_STATUS_* in the public header
     unsigned long long smax[2];  // wavespeed maxima (bit patterns of non-negative doubles), ping-pong by it parity
     FastCoef fc[2];    // FP32 coefficients of dt (fc[0]) and dt/2 (fc[1]), formed by the dt kernel
+    StepRatio xr[2];   // the same ratios in FP64
     double* dt_log;           // non-null: the dt kernel records each step's dt at dt_log[it]
     const double* dt_fixed;   // non-null: step `it` takes dt_fixed[it] instead of the CFL rule
 };
@@ -74,6 +81,47 @@ enum : int {
     ST_TIMEOUT = 4,         // a bounded device wait gave up
     ST_NEGATIVE = 8,        // non-positive density or pressure produced by the FP32 path
 };
+
+// The next step's dt from the last CFL reduction, Solvers/EulerSolvers.cpp:130-161: dt = CFL * (dx / s_max);
+// x0.2 while it <= 5; clamped so that t + dt does not pass t_final.  The solver loop
+// `while (t < t_final)` becomes `active`.  One thread does this between two sweeps of every step, so
+// its latency counts: five FP64 divisions of 565 cycles each one after the other were 1.4 us; the
+// quotients come from the integer pipes (three of about 240 cycles, two of them independent), and
+// those of dt/2 are the ones of dt halved and doubled, which is exact.
+CG_D void step_ctl_advance(StepCtl* c) {
+    const double t = c->t, t_final = c->t_final, dx = c->dx;
+    const int it = c->it;
+    if (!(t < t_final) || it >= c->it_limit) {
+        c->active = 0;
+        c->dt = 0.0;
+        return;
+    }
+    double dt;
+    if (c->dt_fixed) {
+        dt = c->dt_fixed[it];
+    } else {
+        const double smax = __longlong_as_double((long long)c->smax[it & 1]);
+        dt = c->cfl * quotient(dx, smax);
+        if (it <= 5) dt = dt * 0.2;
+        if ((t + dt) > t_final) dt = t_final - t;
+    }
+    if (!(dt > 0.0) || !isfinite(dt)) c->status |= ST_NONFINITE;
+    if (c->dt_log) c->dt_log[it] = dt;
+    c->dt = dt;
+    StepRatio r{xm::div(dt, dx), xm::div(dx, dt)}, h{0.5 * r.d, 2.0 * r.c};
+    if (!xm::finite(r.d + r.c)) {
+        r = make_ratio(dt, dx);
+        h = make_ratio(dt * 0.5, dx);
+    }
+    c->xr[0] = r;
+    c->xr[1] = h;
+    c->fc[0] = FastCoef{(float)r.d, (float)(0.5 * r.d), (float)(0.25 * r.c)};
+    c->fc[1] = FastCoef{(float)h.d, (float)(0.5 * h.d), (float)(0.25 * h.c)};
+    c->active = 1;
+    c->smax[(it + 1) & 1] = 0ull;
+    c->t = t + dt;
+    c->it = it + 1;
+}
 
 // Max of non-negative doubles (ordering of their bit patterns equals numeric ordering).
 // The slot only grows while a kernel reduces into it, so a block whose value does not exceed what

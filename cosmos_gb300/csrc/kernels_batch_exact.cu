@@ -7,21 +7,18 @@ namespace cg {
 
 namespace {
 
-using PE = ExactPolicy<NewtonExact<double>>;
+using PE = ExactPolicy<NewtonExact>;
 
 PE make_exact(const BatchLaunch& L, int axis) {
     PE p;
-    p.sys = NewtonExact<double>{L.gamma, nullptr};
+    p.st = ExactStages<NewtonExact>{NewtonExact(L.gamma), make_bias(L.bias), L.lim};
     p.lm.axis = axis;
     p.lm.nx = 0;
     p.dims = 2;
-    p.order = 2;
     p.ny = 0;
     p.dx = 0.0;
     p.dt = 0.0;
-    p.w = L.bias;
-    p.lim = L.lim;
-    p.capped = 0;
+    p.r = StepRatio{0.0, 0.0};
     return p;
 }
 

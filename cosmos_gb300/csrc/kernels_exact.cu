@@ -1,5 +1,6 @@
 // FP64 reference-exact kernels.  Compiled with --fmad=false so that every double operation is
 // rounded exactly as the reference's (built with -ffp-contract=off) -- results are bit-identical.
+#include "exact_tiles.cuh"
 #include "launch.h"
 #include "policies.cuh"
 
@@ -7,65 +8,65 @@ namespace cg {
 
 namespace {
 
-constexpr int kXThreads = 128;  // X sweep tile: 128 evolutions, 127 fluxes, 126 updates
-constexpr int kYThreads = 64;   // Y sweep: columns per block
-constexpr int kYSeg = 16;       // Y sweep: rows marched per thread
-
 template <class Sys>
 ExactPolicy<Sys> make_policy(const SweepArgs& a, const Sys& sys) {
     ExactPolicy<Sys> p;
-    p.sys = sys;
+    p.st = ExactStages<Sys>{sys, make_bias(a.bias), a.lim};
     p.lm.axis = a.G.axis;
     p.lm.nx = a.G.nx;
     p.dims = a.G.dims;
-    p.order = a.order;
     p.ny = a.G.ny;
     p.dx = a.dx;
     p.dt = 0.0;
-    p.w = a.bias;
-    p.lim = a.lim;
-    p.capped = 0;
+    p.r = StepRatio{0.0, 0.0};
     return p;
 }
 
-template <class Pol>
-cudaError_t run_sweep(const Pol& pol, const SweepArgs& a) {
+TileArgs tile_args(const SweepArgs& a) {
+    return TileArgs{a.G, a.dx, make_bias(a.bias), a.lim, a.order, (const double*)a.src, (double*)a.dst, a.ds, a.out};
+}
+
+template <class Sys, int AXIS, int NT, int LC>
+void run_tiles(const ExactStages<Sys>& S, const SweepArgs& a) {
+    constexpr int T = NT / LC - 2;
     const Geom& G = a.G;
-    const double* src = (const double*)a.src;
-    double* dst = (double*)a.dst;
-    if (G.axis == 0) {
-        dim3 grid((G.nx + kXThreads - 3) / (kXThreads - 2), G.ny);
-        if constexpr (Pol::kShared) {
-            if (a.order == 2) sweep_x_own_kernel<Pol, 2, kXThreads><<<grid, kXThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
-            else sweep_x_own_kernel<Pol, 1, kXThreads><<<grid, kXThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
-        } else {
-            if (a.order == 2) sweep_x_kernel<Pol, 2, kXThreads><<<grid, kXThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
-            else sweep_x_kernel<Pol, 1, kXThreads><<<grid, kXThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
-        }
+    const TileArgs A = tile_args(a);
+    const dim3 grid = AXIS == 0 ? dim3((G.nx + T - 1) / T, G.ny) : dim3((G.nx + LC - 1) / LC, (G.ny + T - 1) / T);
+    if (a.out.mask) {
+        if (a.order == 2) exact_tile_kernel<Sys, AXIS, 2, NT, LC, true><<<grid, NT, 0, a.stream>>>(S, A);
+        else exact_tile_kernel<Sys, AXIS, 1, NT, LC, true><<<grid, NT, 0, a.stream>>>(S, A);
     } else {
-        dim3 grid((G.nx + kYThreads - 1) / kYThreads, (G.ny + kYSeg - 1) / kYSeg);
-        if (a.order == 2) sweep_y_kernel<Pol, 2, kYThreads, kYSeg><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
-        else sweep_y_kernel<Pol, 1, kYThreads, kYSeg><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
+        if (a.order == 2) exact_tile_kernel<Sys, AXIS, 2, NT, LC, false><<<grid, NT, 0, a.stream>>>(S, A);
+        else exact_tile_kernel<Sys, AXIS, 1, NT, LC, false><<<grid, NT, 0, a.stream>>>(S, A);
     }
+}
+
+// X sweeps take one-warp tiles (30 of 32 cells update, against 126 of 128) where the larger ones would not
+// give every SM a block.
+template <class Sys>
+cudaError_t run_sweep(const Sys& sys, const SweepArgs& a) {
+    const ExactStages<Sys> S{sys, make_bias(a.bias), a.lim};
+    if (a.G.axis == 1) run_tiles<Sys, 1, 128, 4>(S, a);
+    else if ((a.G.nx + 125) / 126 * (long long)a.G.ny < device_sm_count()) run_tiles<Sys, 0, 32, 1>(S, a);
+    else run_tiles<Sys, 0, 128, 1>(S, a);
     count_launch();
     return cudaGetLastError();
 }
 
-GRExact make_gr(const SweepArgs& a) {
-    GRExact s;
-    s.g = a.gamma;
-    s.bh = BHExact{a.bh[0], a.bh[1], a.bh[2], a.bh[3], a.bh[4]};
-    s.h = a.dx;
-    s.capped = nullptr;
-    return s;
-}
+GRExact make_gr(const SweepArgs& a, int* status = nullptr) { return GRExact(a.gamma, a.bh, a.dx, status); }
 
 }  // namespace
 
 cudaError_t launch_sweep_exact(const SweepArgs& a) {
-    if (a.system == 0) return run_sweep(make_policy(a, NewtonExact<double>{a.gamma}), a);
-    if (a.system == 1) return run_sweep(make_policy(a, SRExact{a.gamma, nullptr}), a);
-    return run_sweep(make_policy(a, make_gr(a)), a);
+    if (a.system == 0) return run_sweep(NewtonExact(a.gamma), a);
+    if (a.system == 1) return run_sweep(SRExact(a.gamma, a.out.status), a);
+    const GRExact S = make_gr(a, a.out.status);
+    const TileArgs A = tile_args(a);
+    const Geom& G = a.G;
+    if (G.axis == 0) gr_tile_kernel<0, 64, 1><<<dim3((G.nx + 62) / 63, G.ny), 64, 0, a.stream>>>(S, A);
+    else gr_tile_kernel<1, 128, 4><<<dim3((G.nx + 3) / 4, (G.ny + 30) / 31), 128, 0, a.stream>>>(S, A);
+    count_launch();
+    return cudaGetLastError();
 }
 
 cudaError_t launch_wavespeed_exact(const SweepArgs& a, unsigned long long* slot) {
@@ -79,8 +80,8 @@ cudaError_t launch_wavespeed_exact(const SweepArgs& a, unsigned long long* slot)
     int blocks = (int)((n + NT - 1) / NT);
     if (blocks > device_sm_count() * 16) blocks = device_sm_count() * 16;
     const double* src = (const double*)a.src;
-    if (a.system == 0) wavespeed_kernel<ExactPolicy<NewtonExact<double>>, NT><<<blocks, NT, 0, a.stream>>>(make_policy(b, NewtonExact<double>{a.gamma}), b.G, src, o);
-    else if (a.system == 1) wavespeed_kernel<ExactPolicy<SRExact>, NT><<<blocks, NT, 0, a.stream>>>(make_policy(b, SRExact{a.gamma, nullptr}), b.G, src, o);
+    if (a.system == 0) wavespeed_kernel<ExactPolicy<NewtonExact>, NT><<<blocks, NT, 0, a.stream>>>(make_policy(b, NewtonExact(a.gamma)), b.G, src, o);
+    else if (a.system == 1) wavespeed_kernel<ExactPolicy<SRExact>, NT><<<blocks, NT, 0, a.stream>>>(make_policy(b, SRExact(a.gamma)), b.G, src, o);
     else wavespeed_kernel<ExactPolicy<GRExact>, NT><<<blocks, NT, 0, a.stream>>>(make_policy(b, make_gr(a)), b.G, src, o);
     count_launch();
     return cudaGetLastError();
@@ -90,57 +91,74 @@ cudaError_t launch_wavespeed_exact(const SweepArgs& a, unsigned long long* slot)
 // Solvers/BlackHoleEulerForcingSolver.cpp:187-250: per cell away from the horizon (cell and its
 // 2 (1D) or 4 (2D) neighbours outside), conserved neighbours from a 1-ghost transmissive copy,
 // classical RK4 with interleaved fractional sweeps, converted back at the cell.
-__global__ void __launch_bounds__(128) rk_source_kernel(GRExact sys, Geom G, double dx, double w, int lim,
-                                                        const double* __restrict__ src, double* __restrict__ dst,
-                                                        DtSrc ds, int* status) {
+// Cell (j, i) of the grid and its neighbours' coordinates, each index times dx as the reference has them.
+struct RkAt {
+    int j, i;
+    double dx;
+    CG_D Pt at(int dj, int di) const { return Pt{(j + dj) * dx, (i + di) * dx, 0.0}; }
+};
+struct RkCell { V5<double> c[5]; };  // primitives of the left, right, top and bottom neighbours and of the cell
+template <class T>
+CG_D V5<T> rk_source_cell(const GRExact* S, int dims, const RkCell& c, RkAt a, double dt, const StepRatio& sr,
+                          const Bias& w, int lim) {
+    V5<T> u[5];
+    Metric<T> g;
+#pragma unroll 1
+    for (int n = 0; n < 5; n++) {
+        if (dims == 1 && (n == 2 || n == 3)) continue;
+        V5<T> p;
+#pragma unroll
+        for (int f = 0; f < 5; f++) p.v[f] = T(c.c[n].v[f]);
+        gr_metric(S, a.at(n == 0 ? -1 : n == 1 ? 1 : 0, n == 2 ? -1 : n == 3 ? 1 : 0), &g);
+        u[n] = gr_cons(S, &g, p);
+    }
+    const V5<T> nc = rk_cell_exact(S, dims, u, a.at(0, 0), a.dx, dt, sr, w, lim, &g);
+    return gr_prim(S, &g, nc);
+}
+__device__ __noinline__ V5<double> slow_rk(GRExact S, int dims, RkCell c, RkAt a, double dt, StepRatio sr, Bias w, int lim) {
+    return rk_source_cell<double>(&S, dims, c, a, dt, sr, w, lim);
+}
+
+__global__ void __launch_bounds__(64) rk_source_kernel(const __grid_constant__ GRExact sys, Geom G, double dx, Bias w,
+                                                       int lim, const double* __restrict__ src, double* __restrict__ dst,
+                                                       DtSrc ds) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;
     if (j >= G.nx) return;
     const size_t idx = (size_t)i * G.pitch + j;
     double dt;
-    int capped = 0;
-    sys.capped = &capped;
-    bool on = ds.get(dt);
-    const BHExact& b = sys.bh;
-    if (on) {
-        if (G.dims == 1)
-            on = !b.excised(j * dx, 0.0, 0.0) && !b.excised((j - 1) * dx, 0.0, 0.0) && !b.excised((j + 1) * dx, 0.0, 0.0);
-        else
-            on = !b.excised(j * dx, i * dx, 0.0) && !b.excised((j - 1) * dx, i * dx, 0.0) &&
-                 !b.excised((j + 1) * dx, i * dx, 0.0) && !b.excised(j * dx, (i - 1) * dx, 0.0) &&
-                 !b.excised(j * dx, (i + 1) * dx, 0.0);
-    }
-    if (!on) {
+    if (!ds.get(dt) || gr_excised_near(sys.bh, G.dims, i, j, dx, 1)) {
 #pragma unroll
         for (int f = 0; f < 5; f++) dst[f * G.fstride + idx] = src[f * G.fstride + idx];
         return;
     }
-    auto ld = [&](int ii, int jj, double* p) {
+    auto ld = [&](int ii, int jj, V5<double>& p) {
         const size_t k = (size_t)ghost_index(ii, G.ny, 0) * G.pitch + ghost_index(jj, G.nx, 0);
 #pragma unroll
-        for (int f = 0; f < 5; f++) p[f] = src[f * G.fstride + k];
+        for (int f = 0; f < 5; f++) p.v[f] = src[f * G.fstride + k];
     };
-    double p[5], cl[5], cm[5], cr[5], ct[5], cb[5], nc[5];
-    const double y = G.dims == 1 ? 0.0 : i * dx;
-    const Pt q{j * dx, y, 0.0};
-    ld(i, j - 1, p); sys.cons(p, Pt{(j - 1) * dx, y, 0.0}, cl);
-    ld(i, j, p); sys.cons(p, q, cm);
-    ld(i, j + 1, p); sys.cons(p, Pt{(j + 1) * dx, y, 0.0}, cr);
+    RkCell c;
+    ld(i, j - 1, c.c[0]);
+    ld(i, j + 1, c.c[1]);
     if (G.dims == 2) {
-        ld(i - 1, j, p); sys.cons(p, Pt{j * dx, (i - 1) * dx, 0.0}, ct);
-        ld(i + 1, j, p); sys.cons(p, Pt{j * dx, (i + 1) * dx, 0.0}, cb);
+        ld(i - 1, j, c.c[2]);
+        ld(i + 1, j, c.c[3]);
     }
-    rk_cell_exact(sys, G.dims, cl, cm, cr, ct, cb, q, dx, dt, w, lim, nc);
-    sys.prim(nc, q, p);
+    ld(i, j, c.c[4]);
+    const RkAt at{j, G.dims == 1 ? 0 : i, dx};
+    const StepRatio sr = ds.ratio(dt, dx);
+    const V5<xd> nc = rk_source_cell<xd>(&sys, G.dims, c, at, dt, sr, w, lim);
+    V5<double> o;
+    store5(nc.v, o.v);
+    if (any_nonfinite(nc.v, 5)) o = slow_rk(sys, G.dims, c, at, dt, sr, w, lim);
 #pragma unroll
-    for (int f = 0; f < 5; f++) dst[f * G.fstride + idx] = p[f];
-    if (capped && status) atomicOr(status, ST_NEWTON_CAP);
+    for (int f = 0; f < 5; f++) dst[f * G.fstride + idx] = o.v[f];
 }
 
 cudaError_t launch_rk_source_exact(const SweepArgs& a) {
-    dim3 grid((a.G.nx + 127) / 128, a.G.ny);
-    rk_source_kernel<<<grid, 128, 0, a.stream>>>(make_gr(a), a.G, a.dx, a.bias, a.lim, (const double*)a.src,
-                                                 (double*)a.dst, a.ds, a.out.status);
+    dim3 grid((a.G.nx + 63) / 64, a.G.ny);
+    rk_source_kernel<<<grid, 64, 0, a.stream>>>(make_gr(a, a.out.status), a.G, a.dx, make_bias(a.bias), a.lim,
+                                                (const double*)a.src, (double*)a.dst, a.ds);
     count_launch();
     return cudaGetLastError();
 }
@@ -178,33 +196,8 @@ cudaError_t launch_prim_out_exact(const void* soa, double* aos, const Geom& G, c
 }
 
 // ------------------------------------------------------------------ step controller
-// Solvers/EulerSolvers.cpp:130-161: dt = CFL * (dx / s_max); x0.2 while it <= 5; clamped so
-// that t + dt does not pass t_final.  The solver loop `while (t < t_final)` becomes `active`.
 __global__ void dt_kernel(StepCtl* c) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (!(c->t < c->t_final) || c->it >= c->it_limit) {
-        c->active = 0;
-        c->dt = 0.0;
-        return;
-    }
-    double dt;
-    if (c->dt_fixed) {
-        dt = c->dt_fixed[c->it];
-    } else {
-        const double smax = __longlong_as_double((long long)c->smax[c->it & 1]);
-        dt = c->cfl * (c->dx / smax);
-        if (c->it <= 5) dt = dt * 0.2;
-        if ((c->t + dt) > c->t_final) dt = c->t_final - c->t;
-    }
-    if (!(dt > 0.0) || !isfinite(dt)) c->status |= ST_NONFINITE;
-    if (c->dt_log) c->dt_log[c->it] = dt;
-    c->dt = dt;
-    c->fc[0] = make_fast_coef(dt, c->dx);
-    c->fc[1] = make_fast_coef(dt * 0.5, c->dx);
-    c->active = 1;
-    c->smax[(c->it + 1) & 1] = 0ull;
-    c->t = c->t + dt;
-    c->it = c->it + 1;
+    if (threadIdx.x == 0 && blockIdx.x == 0) step_ctl_advance(c);
 }
 cudaError_t launch_dt_kernel(StepCtl* ctl, cudaStream_t st) {
     dt_kernel<<<1, 32, 0, st>>>(ctl);
@@ -220,7 +213,7 @@ struct ConsLoader {
     int system, precision;
     Geom G;
     const void* state;
-    NewtonExact<double> nw;
+    NewtonExact nw;
     SRExact sr;
     GRExact gr;
     CG_D void get(int i, int j, Pt q, double* u) const {
@@ -312,8 +305,8 @@ static ConsLoader make_loader(const SweepArgs& a, int precision, const void* sta
     L.precision = precision;
     L.G = G;
     L.state = state;
-    L.nw = NewtonExact<double>{a.gamma};
-    L.sr = SRExact{a.gamma, nullptr};
+    L.nw = NewtonExact(a.gamma);
+    L.sr = SRExact(a.gamma);
     L.gr = make_gr(a);
     return L;
 }
@@ -529,7 +522,7 @@ CG_D void gr_eigenvalues(const GRExact& S, const double* p, Pt q, double* o) {
     double gm[9], gs[9];
     S.bh.gamma(q.x, q.y, q.z, gm);
     inverse3(gm, gs);
-    const double cs = sr_sound(p[0], p[4], S.g);
+    const double cs = sr_sound(p[0], p[4], S.k);
     const double v[3] = {p[1], p[2], p[3]};
     double v2 = 0.0;
     for (int i = 0; i < 3; i++)
@@ -543,7 +536,7 @@ CG_D void gr_eigenvalues(const GRExact& S, const double* p, Pt q, double* o) {
     }
 }
 
-__global__ void state_eval_kernel(StateEvalArgs a, NewtonExact<double> nw, SRExact sr, GRExact gr) {
+__global__ void state_eval_kernel(StateEvalArgs a, NewtonExact nw, SRExact sr, const __grid_constant__ GRExact gr) {
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.n; k += (size_t)gridDim.x * blockDim.x) {
         const double* v = a.in + a.in_stride * k;
         double* o = a.out + a.out_stride * k;
@@ -560,7 +553,7 @@ __global__ void state_eval_kernel(StateEvalArgs a, NewtonExact<double> nw, SRExa
                 break;
             case kStateSound:  // Euler/EulerEquationOfState.cpp:17-22; SR :10-18; black hole :519-549
                 if (a.system == 0) o[0] = sqrt((g * v[4]) / v[0]);
-                else if (a.system == 1) o[0] = sr_sound(v[0], v[4], g);
+                else if (a.system == 1) o[0] = sr_sound(v[0], v[4], sr.k);
                 else o[0] = gr.sound_speed(v, q);
                 break;
             case kStateInternalEnergy:  // Euler/EulerEquationOfState.cpp:3-8
@@ -576,7 +569,7 @@ __global__ void state_eval_kernel(StateEvalArgs a, NewtonExact<double> nw, SRExa
                 o[0] = (v[4] * (g - 1.0)) * v[0];
                 break;
             case kStateEnthalpy:  // RelativisticEuler/RelativisticEulerEquationOfState.cpp:3-8
-                o[0] = sr_enthalpy(v[0], v[4], g);
+                o[0] = sr_enthalpy(v[0], v[4], sr.k);
                 break;
             case kStateSource:  // BlackHoleEuler/BlackHoleEulerStateVector.cpp:359-510
                 gr.source(v, q, o);
@@ -591,7 +584,7 @@ __global__ void state_eval_kernel(StateEvalArgs a, NewtonExact<double> nw, SRExa
                 o[0] = limiter_exact(v[0], a.bias, a.lim);
                 break;
             case kStateSlope:  // Solvers/SlopeLimiters.cpp:71-101 on three conserved vectors
-                slope_exact(v, v + 5, v + 10, a.bias, a.lim, o);
+                slope_exact(v, v + 5, v + 10, make_bias(a.bias), a.lim, o);
                 break;
             default:
                 break;
@@ -602,8 +595,8 @@ __global__ void state_eval_kernel(StateEvalArgs a, NewtonExact<double> nw, SRExa
 cudaError_t launch_state_eval(const SweepArgs& s, const StateEvalArgs& a) {
     size_t b = (a.n + 127) / 128;
     if (b > device_sm_count() * 8) b = device_sm_count() * 8;
-    state_eval_kernel<<<(int)(b ? b : 1), 128, 0, s.stream>>>(a, NewtonExact<double>{s.gamma, nullptr},
-                                                                SRExact{s.gamma, nullptr}, make_gr(s));
+    state_eval_kernel<<<(int)(b ? b : 1), 128, 0, s.stream>>>(a, NewtonExact(s.gamma),
+                                                                SRExact(s.gamma), make_gr(s));
     count_launch();
     return cudaGetLastError();
 }
@@ -632,6 +625,8 @@ CG_D void iface_item(const Sys& S, bool gr, const IfaceArgs& A, const double* a,
     const int op = A.op;
     const int axis = (op & 1) ? 1 : 0;
     const double dx = A.dx, dt = A.dt;
+    const StepRatio sr = make_ratio(dt, dx);
+    const Bias w = make_bias(A.bias);
     switch (op) {
         case 0: { const double r = dx / dt; for (int k = 0; k < 5; k++) o[k] = 0.5 * ((c[k] + d[k]) + (r * (a[k] - b[k]))); break; }
         case 1: { const double r = dt / dx; for (int k = 0; k < 5; k++) o[k] = 0.5 * ((a[k] + b[k]) + (r * (c[k] - d[k]))); break; }
@@ -660,16 +655,16 @@ CG_D void iface_item(const Sys& S, bool gr, const IfaceArgs& A, const double* a,
             S.flux(us, axis, q, o);
             break;
         }
-        case 10: case 11: force_exact(S, a, b, q, axis, dx, dt, o); break;
+        case 10: case 11: force_exact(S, a, b, q, axis, dx, sr, o); break;
         case 12: case 13: {
             double eR[5], eL[5];
-            evolve_half_exact(S, a, b, c, shift_pt(q, axis, -(dx * 0.5)), axis, dx, dt, A.bias, A.lim, (double*)nullptr, eR);
-            evolve_half_exact(S, b, c, d, shift_pt(q, axis, dx * 0.5), axis, dx, dt, A.bias, A.lim, eL, (double*)nullptr);
-            force_exact(S, eR, eL, q, axis, dx, dt, o);
+            evolve_half_exact(S, a, b, c, shift_pt(q, axis, -(dx * 0.5)), axis, dx, sr, w, A.lim, (double*)nullptr, eR);
+            evolve_half_exact(S, b, c, d, shift_pt(q, axis, dx * 0.5), axis, dx, sr, w, A.lim, eL, (double*)nullptr);
+            force_exact(S, eR, eL, q, axis, dx, sr, o);
             break;
         }
         case 14: case 15:
-            evolve_half_exact(S, a, b, c, q, axis, dx, dt, A.bias, A.lim, A.side == 0 ? o : nullptr,
+            evolve_half_exact(S, a, b, c, q, axis, dx, sr, w, A.lim, A.side == 0 ? o : nullptr,
                               A.side == 0 ? nullptr : o);
             break;
         case 16: case 17: {
@@ -683,7 +678,7 @@ CG_D void iface_item(const Sys& S, bool gr, const IfaceArgs& A, const double* a,
     }
 }
 
-__global__ void iface_kernel(IfaceArgs A, NewtonExact<double> nw, SRExact sr, GRExact gr) {
+__global__ void iface_kernel(IfaceArgs A, NewtonExact nw, SRExact sr, const __grid_constant__ GRExact gr) {
     const int w = A.width;
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < A.n; k += (size_t)gridDim.x * blockDim.x) {
         const double* a = A.in + (size_t)w * k;
@@ -692,15 +687,23 @@ __global__ void iface_kernel(IfaceArgs A, NewtonExact<double> nw, SRExact sr, GR
         if (A.system == 0) iface_item(nw, false, A, a, q, o);
         else if (A.system == 1) iface_item(sr, false, A, a, q, o);
         else if (A.op <= 17) iface_item(gr, true, A, a, q, o);
-        else if (A.op <= 19) evolve_fraction_exact(gr, A.frac, a, a + 5, a + 10, q, A.op - 18, A.dx, A.dt, A.bias, A.lim, o);
+        else if (A.op <= 19) evolve_fraction_exact(gr, A.frac, a, a + 5, a + 10, q, A.op - 18, A.dx, make_ratio(A.dt, A.dx), make_bias(A.bias), A.lim, o);
         else if (A.op == 20) {
             double u[5];
             for (int f = 0; f < 5; f++) u[f] = a[f] + a[5 + f];
             gr.prim(u, q, o);
-        } else if (A.op == 21) {
-            rk_cell_exact(gr, 1, a, a + 5, a + 10, a, a, q, A.dx, A.dt, A.bias, A.lim, o);
-        } else {
-            rk_cell_exact(gr, 2, a, a + 5, a + 10, a + 15, a + 20, q, A.dx, A.dt, A.bias, A.lim, o);
+        } else {  // 21: left, middle, right; 22: left, middle, right, top, bottom
+            const int dims = A.op - 20;
+            V5<double> u[5];
+            Metric<double> g;
+            for (int f = 0; f < 5; f++) {
+                u[0].v[f] = a[f];
+                u[4].v[f] = a[5 + f];
+                u[1].v[f] = a[10 + f];
+                u[2].v[f] = dims == 2 ? a[15 + f] : 0.0;
+                u[3].v[f] = dims == 2 ? a[20 + f] : 0.0;
+            }
+            give(rk_cell_exact(&gr, dims, u, q, A.dx, A.dt, make_ratio(A.dt, A.dx), make_bias(A.bias), A.lim, &g), o);
         }
     }
 }
@@ -710,7 +713,7 @@ cudaError_t launch_interface_eval(const SweepArgs& s, const IfaceArgs& a) {
     if (b > (size_t)device_sm_count() * 8) b = (size_t)device_sm_count() * 8;
     SweepArgs g = s;
     g.dx = a.dx;  // the black-hole metric derivatives take the cell spacing (the reference's h)
-    iface_kernel<<<(int)(b ? b : 1), 128, 0, s.stream>>>(a, NewtonExact<double>{s.gamma, nullptr}, SRExact{s.gamma, nullptr},
+    iface_kernel<<<(int)(b ? b : 1), 128, 0, s.stream>>>(a, NewtonExact(s.gamma), SRExact(s.gamma),
                                                          make_gr(g));
     count_launch();
     return cudaGetLastError();
@@ -720,12 +723,12 @@ cudaError_t launch_interface_eval(const SweepArgs& s, const IfaceArgs& a) {
 // Every public quantity of the reference's BlackHoleSpacetime (BlackHoleEuler/BlackHoleSpacetime.cpp:
 // 54-386) at one point, metric derivatives by the reference's centred differences with spacing
 // S.h, in the layout of the public COSMOS_ST_* offsets.
-__global__ void spacetime_kernel(GRExact S, size_t n, const double* __restrict__ xyz, double* __restrict__ out) {
+__global__ void spacetime_kernel(const __grid_constant__ GRExact S, size_t n, const double* __restrict__ xyz, double* __restrict__ out) {
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
         const Pt q{xyz[3 * k], xyz[3 * k + 1], xyz[3 * k + 2]};
         double* o = out + (size_t)kSpacetimeWidth * k;
         const BHExact& b = S.bh;
-        o[0] = b.H(q.x, q.y, q.z);                            // computeKerrSchildScalar
+        o[0] = b.H<double>(q.x, q.y, q.z);                            // computeKerrSchildScalar
         b.l(q.x, q.y, q.z, o + 1);                            // computeKerrSchildVector
         b.L4(q.x, q.y, q.z, o + 4);                           // computeKerrSchildSpacetimeVector
         const double h = S.h, hs = 0.5 * h;

@@ -11,14 +11,7 @@ namespace cg {
 
 namespace {
 
-GRExact make_gr_exact(const SweepArgs& a) {
-    GRExact s;
-    s.g = a.gamma;
-    s.bh = BHExact{a.bh[0], a.bh[1], a.bh[2], a.bh[3], a.bh[4]};
-    s.h = a.dx;
-    s.capped = nullptr;
-    return s;
-}
+GRExact make_gr_exact(const SweepArgs& a) { return GRExact(a.gamma, a.bh, a.dx); }
 
 // ---------------------------------------------------------------- metric tables (FP64 -> FP32)
 // Point (i, j) of a table at x = (j + xo) dx, y = (i + yo) dx (y = 0 on 1D grids), with xo, yo
@@ -123,7 +116,6 @@ struct GRFastPolicy {
     using Cell = V5<float>;
     using Face = V5<float>;
     using Coef = FastCoef;
-    static constexpr bool kShared = true;
     static constexpr bool kMasked = true;  // excision: cells with an excised stencil keep their state
     static constexpr bool kHasDx = false;
     NewtonFastParams NP;
@@ -158,7 +150,6 @@ struct GRFastPolicy {
         gr_evolve_fast<AXIS, LIM>(P, NP, l.v, m.v, r.v, center(line, k - 1), center(line, k), center(line, k + 1),
                                   face(line, k), face(line, k + 1), half_dtdx, L.v, R.v, &flags);
     }
-    CG_D void recon_side(const Cell&, const Cell&, const Cell&, int, int, int, Face&) const {}
     CG_D void face_of(const Cell& c, Face& f) const { f = c; }
     CG_D void flux(const Face& L, const Face& R, int line, int f, V5<float>& F) {
         gr_force_fast<AXIS>(P, L.v, R.v, center(line, f - 1), face(line, f), center(line, f), half_dtdx, q_dxdt, F.v,

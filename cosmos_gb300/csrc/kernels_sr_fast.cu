@@ -43,9 +43,8 @@ void run_lim(const SweepArgs& a) {
 
 // Primitive (double, AoS) -> conserved FP32 SoA with the reference's FP64 formula
 // (RelativisticEuler/RelativisticEulerStateVector.cpp:116-136), rounded once.
-__global__ void sr_prim_in_kernel(const double* __restrict__ aos, float* __restrict__ soa, Geom G, double gamma) {
+__global__ void sr_prim_in_kernel(const double* __restrict__ aos, float* __restrict__ soa, Geom G, SRExact S) {
     const size_t n = (size_t)G.nx * G.ny;
-    SRExact S{gamma, nullptr};
     for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
         const size_t i = c / G.nx, j = c % G.nx;
         double u[5];
@@ -55,9 +54,8 @@ __global__ void sr_prim_in_kernel(const double* __restrict__ aos, float* __restr
     }
 }
 // Conserved FP32 -> primitives with the reference's full FP64 recovery.
-__global__ void sr_prim_out_kernel(const float* __restrict__ soa, double* __restrict__ aos, Geom G, double gamma) {
+__global__ void sr_prim_out_kernel(const float* __restrict__ soa, double* __restrict__ aos, Geom G, SRExact S) {
     const size_t n = (size_t)G.nx * G.ny;
-    SRExact S{gamma, nullptr};
     for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
         const size_t i = c / G.nx, j = c % G.nx;
         double u[5];
@@ -97,12 +95,12 @@ cudaError_t launch_wavespeed_sr_fast(const SweepArgs& a, unsigned long long* slo
 }
 
 cudaError_t launch_prim_in_sr_fast(const double* aos, void* soa, const Geom& G, double gamma, cudaStream_t st) {
-    sr_prim_in_kernel<<<grid_for((size_t)G.nx * G.ny), 256, 0, st>>>(aos, (float*)soa, G, gamma);
+    sr_prim_in_kernel<<<grid_for((size_t)G.nx * G.ny), 256, 0, st>>>(aos, (float*)soa, G, SRExact(gamma));
     count_launch();
     return cudaGetLastError();
 }
 cudaError_t launch_prim_out_sr_fast(const void* soa, double* aos, const Geom& G, double gamma, cudaStream_t st) {
-    sr_prim_out_kernel<<<grid_for((size_t)G.nx * G.ny), 256, 0, st>>>((const float*)soa, aos, G, gamma);
+    sr_prim_out_kernel<<<grid_for((size_t)G.nx * G.ny), 256, 0, st>>>((const float*)soa, aos, G, SRExact(gamma));
     count_launch();
     return cudaGetLastError();
 }

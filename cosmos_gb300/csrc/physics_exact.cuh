@@ -1,9 +1,12 @@
 // Reference-exact device physics.  Every expression keeps the reference's evaluation order
 // (left-to-right C++ semantics of the cited lines), so that a translation unit compiled with
-// --fmad=false produces the reference's FP64 results bit for bit.  Used by the FP64 ("plain
-// FP64") path; also instantiated in FP32 for the SR/GR bulk paths where noted.
+// --fmad=false produces the reference's FP64 results bit for bit.  The functions are generic over
+// the number type T: double (hardware FP64) or xd (exact_math.cuh: products, quotients and roots on
+// the integer pipes, NaN where an operand leaves their range).  A stage whose xd results are not all
+// finite is formed again in double; both give the reference's bits.
 #pragma once
 #include "device_common.cuh"
+#include "exact_math.cuh"
 
 namespace cg {
 
@@ -27,65 +30,111 @@ template <class T> CG_D T limiter_exact(T r, T w, int lim) {
     return mn(T(1.0), gradient_ratio(r, w));
 }
 
-// Solvers/SlopeLimiters.cpp:71-101 (numerator and denominator each clamped to +1e-5)
-template <class T> CG_D void slope_exact(const T* ul, const T* uc, const T* ur, T w, int lim, T* s) {
-    T dl[5], dr[5];
-#pragma unroll
-    for (int k = 0; k < 5; k++) { dl[k] = uc[k] - ul[k]; dr[k] = ur[k] - uc[k]; }
-    const T a = T(0.5) * (T(1.0) + w), b = T(0.5) * (T(1.0) - w);
-#pragma unroll
-    for (int k = 0; k < 5; k++) s[k] = (a * dl[k]) + (b * dr[k]);
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        T num = dl[k], den = dr[k];
-        if (fabs(num) < T(1e-5)) num = T(1e-5);
-        if (fabs(den) < T(1e-5)) den = T(1e-5);
-        s[k] = s[k] * limiter_exact(num / den, w, lim);
+// The bias w and what the slopes take from it, formed once on the host (or per item).
+struct Bias {
+    double w, a, b;  // w, 0.5 (1 + w), 0.5 (1 - w)
+};
+CG_HD Bias make_bias(double w) { return Bias{w, 0.5 * (1.0 + w), 0.5 * (1.0 - w)}; }
+
+// One component of the slope vector, Solvers/SlopeLimiters.cpp:71-101: numerator and denominator each
+// clamped to +1e-5.
+CG_D double limited_slope(double dl, double dr, const Bias& w, int lim) {
+    const double s = (w.a * dl) + (w.b * dr);
+    double num = dl, den = dr;
+    if (fabs(num) < 1e-5) num = 1e-5;
+    if (fabs(den) < 1e-5) den = 1e-5;
+    return s * limiter_exact(num / den, w.w, lim);
+}
+// The same value with the limiter's comparisons on bit patterns and, for bias 0 (every driver's), at
+// most one quotient after r = num / den: with w = 0 both candidates of a minimum have the denominator
+// 1 + r, and rounding is monotone, so the minimum of the rounded quotients is the rounded quotient of
+// the smaller numerator (van Leer 2 min(r, 1) / (1 + r); SuperBee and MinBee 2 / (1 + r) from r = 1
+// on).  Both differences inside the clamp (uniform flow, a velocity that is zero everywhere) give
+// r = 1 and a limiter of 1.
+CG_D xd limited_slope(xd dl, xd dr, const Bias& w, int lim) {
+    const bool plain = w.w == 0.0;
+    const xd s = plain ? half(dl) + half(dr) : (xd(w.a) * dl) + (xd(w.b) * dr);
+    const bool tl = nearer_zero(dl, 1e-5), tr = nearer_zero(dr, 1e-5);
+    if (tl && tr && plain) return s;
+    const xd r = (tl ? xd(1e-5) : dl) / (tr ? xd(1e-5) : dr);
+    if (xm::plain_negative(r.v)) return xm::finite(s.v) ? xd(xm::double_of(xm::bits_of(s.v) & 0x8000000000000000ull)) : s;
+    if (!xm::plain_positive(r.v)) return xd(xm::double_of(0x7ff8000000000000ull));
+    const bool lt1 = below(r, 1.0);
+    if (plain) {
+        xd phi = xd(2.0);
+        bool quotient = true;
+        if (lim == 1) {
+            if (lt1) phi = twice(r);
+        } else if (lt1) {
+            quotient = false;
+            phi = lim == 0 ? (below(r, 0.5) ? twice(r) : xd(1.0)) : r;
+        }
+        if (quotient) phi = phi / (xd(1.0) + r);
+        return s * phi;
     }
+    const xd xi = xd(2.0) / (xd(1.0 - w.w) + (xd(1.0 + w.w) * r));
+    if (!xm::finite(xi.v)) return xi;  // a comparison would lose the NaN
+    xd phi;
+    if (lim == 1) phi = twice(r) / (xd(1.0) + r);
+    else if (lt1) return s * (lim == 0 ? (below(r, 0.5) ? twice(r) : xd(1.0)) : r);
+    else phi = lim == 0 ? r : xd(1.0);
+    if (xi.v < phi.v) phi = xi;
+    if (lim == 0 && 2.0 < phi.v) phi = xd(2.0);
+    return s * phi;
+}
+template <class T> CG_D void slope_exact(const T* ul, const T* uc, const T* ur, const Bias& w, int lim, T* s) {
+#pragma unroll
+    for (int k = 0; k < 5; k++) s[k] = limited_slope(uc[k] - ul[k], ur[k] - uc[k], w, lim);
 }
 
 // ============================================================== Newtonian Euler
-template <class T> struct NewtonExact {
-    T g;
-    int* capped;  // unused (no iterative solve); keeps the policy interface uniform
+struct NewtonExact {
+    double g, g1;  // gamma, gamma - 1
     static constexpr bool kCoords = false;
+    NewtonExact() = default;
+    explicit NewtonExact(double gamma, int* = nullptr) : g(gamma), g1(gamma - 1.0) {}
     // Euler/EulerStateVector.cpp:55-66, computeTotalEnergy :129-134, EoS Euler/EulerEquationOfState.cpp:3-8
-    CG_D void cons(const T* p, Pt, T* u) const {
+    template <class T> CG_D void cons(const T* p, Pt, T* u) const {
         T rho = p[0], vx = p[1], vy = p[2], vz = p[3];
         u[0] = rho; u[1] = rho * vx; u[2] = rho * vy; u[3] = rho * vz;
         T v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
-        T e = p[4] / ((g - T(1.0)) * rho);
-        u[4] = rho * ((T(0.5) * v2) + e);
+        T e = p[4] / (T(g1) * rho);
+        u[4] = rho * (half(v2) + e);
     }
     // Euler/EulerStateVector.cpp:30-40, computePressure Euler/EulerEquationOfState.cpp:10-15
-    CG_D void prim(const T* u, Pt, T* p) const {
+    template <class T> CG_D void prim(const T* u, Pt, T* p) const {
         T rho = u[0];
-        T vx = u[1] / rho, vy = u[2] / rho, vz = u[3] / rho;
+        const auto d = divisor(rho);
+        T vx = u[1] / d, vy = u[2] / d, vz = u[3] / d;
         T v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
-        T e = (u[4] / rho) - (T(0.5) * v2);
-        p[0] = rho; p[1] = vx; p[2] = vy; p[3] = vz; p[4] = (e * (g - T(1.0))) * rho;
+        T e = (u[4] / d) - half(v2);
+        p[0] = rho; p[1] = vx; p[2] = vy; p[3] = vz; p[4] = (e * T(g1)) * rho;
     }
     // Euler/EulerStateVector.cpp:68-89 (x) and :96-117 (y)
-    CG_D void flux(const T* u, int axis, Pt, T* f) const {
+    template <class T> CG_D void flux(const T* u, int axis, Pt, T* f) const {
         T rho = u[0];
-        T vx = u[1] / rho, vy = u[2] / rho, vz = u[3] / rho;
-        T v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
-        T et = u[4] / rho;
-        T pr = ((et - (T(0.5) * v2)) * (g - T(1.0))) * rho;
-        if (axis == 0) {
-            f[0] = rho * vx; f[1] = (rho * (vx * vx)) + pr; f[2] = rho * (vx * vy); f[3] = rho * (vx * vz);
-            f[4] = (rho * (vx * et)) + (vx * pr);
-        } else {
-            f[0] = rho * vy; f[1] = rho * (vy * vx); f[2] = (rho * (vy * vy)) + pr; f[3] = rho * (vy * vz);
-            f[4] = (rho * (vy * et)) + (vy * pr);
-        }
+        const auto d = divisor(rho);
+        T vx = u[1] / d, vy = u[2] / d, vz = u[3] / d;
+        T xx = vx * vx, yy = vy * vy;
+        T v2 = (xx + yy) + (vz * vz);
+        T et = u[4] / d;
+        T pr = ((et - half(v2)) * T(g1)) * rho;
+        // products of two velocities commute exactly, so one form serves both axes
+        const T vn = axis == 0 ? vx : vy;
+        f[0] = rho * vn;
+        const T nn = (rho * (axis == 0 ? xx : yy)) + pr, xy = rho * (vx * vy);
+        f[1] = axis == 0 ? nn : xy;
+        f[2] = axis == 0 ? xy : nn;
+        f[3] = rho * (vn * vz);
+        f[4] = (rho * (vn * et)) + (vn * pr);
     }
     // Solvers/EulerSolvers.cpp:87-128 with Euler/EulerEquationOfState.cpp:17-22;
     // 2D is max(|vx|, |vy| + c) exactly as written at :117-118.
-    CG_D T wavespeed(const T* p, int dims, Pt) const {
-        T c = fabs(sqrt((g * p[4]) / p[0]));
-        if (dims == 1) return fabs(p[1]) + c;
-        return mx(fabs(p[1]), fabs(p[2]) + c);
+    template <class T> CG_D T wavespeed(const T* p, int dims, Pt) const {
+        T c = magnitude(root((T(g) * p[4]) / p[0]));
+        if (hopeless(c)) return c;  // a maximum would drop it
+        if (dims == 1) return magnitude(p[1]) + c;
+        return larger(magnitude(p[1]), magnitude(p[2]) + c);
     }
 };
 
@@ -94,195 +143,234 @@ template <class T> struct NewtonExact {
 // functions (:138-309) and, on densitised variables, BlackHoleEuler/BlackHoleEulerStateVector.cpp
 // (:30-103, :159-350 with tol 1e-10 in the x flux at :205, :359-430).  Newton from x = 1 on the
 // quartic in x, stop when |x - x_new| < tol keeping the previous iterate, at most 1000 steps.
-struct C2P { double rho, vx, vy, vz, p, W, h; };
+template <class T> struct C2P { T rho, vx, vy, vz, p, W, h; };
+// what the solve takes from gamma, formed once on the host
+struct GammaConst {
+    double g, cst, lin, quad, gm, gm4, hg;
+    GammaConst() = default;
+    // hg: gamma / (gamma - 1), the enthalpy's factor
+    explicit GammaConst(double g_) : g(g_), cst(-1.0 / (g_ * g_)), lin((g_ - 1.0) / (g_ * g_)), quad((g_ - 2.0) / g_),
+                                     gm((g_ - 1.0) / g_), gm4(4.0 * ((g_ - 1.0) / g_)), hg(g_ / (g_ - 1.0)) {}
+};
 
-CG_D C2P con2prim_exact(double D, double Sx, double Sy, double Sz, double tau, double g, double tol, int* capped) {
-    double q = ((tau + D) * (tau + D)) - (((Sx * Sx) + (Sy * Sy)) + (Sz * Sz));
-    double dc = D / sqrt(q);
-    double ec = (D + tau) / sqrt(q);
-    if (q < 1e-8) {
-        dc = D / sqrt(1e-8);
-        ec = (D + tau) / sqrt(1e-8);
-    }
-    double constant = -1.0 / (g * g);
-    double linear = (-2.0 * dc) * ((g - 1.0) / (g * g));
-    double quadratic = ((((g - 2.0) / g) * ((ec * ec) - 1.0)) + 1.0) - (((dc * dc) * ((g - 1.0) / g)) * ((g - 1.0) / g));
-    double quartic = (ec * ec) - 1.0;
-    double eta = (2.0 * dc) * ((g - 1.0) / g);
-    double x = 1.0;
+// One copy per number type (out of line): a sweep recovers eight states per cell, and the iteration
+// is thousands of cycles long.  status: ST_NEWTON_CAP is set there when the cap is reached (may be null).
+template <class T>
+__device__ __noinline__ C2P<T> con2prim_exact(V5<T> u, GammaConst k, double tol, int* status) {
+    const T D = u.v[0], Sx = u.v[1], Sy = u.v[2], Sz = u.v[3], tau = u.v[4];
+    const T E = tau + D;
+    T q = (E * E) - (((Sx * Sx) + (Sy * Sy)) + (Sz * Sz));
+    const bool tiny = below(q, 1e-8);
+    const auto dq = divisor(root(tiny ? T(1e-8) : q));
+    const T dc = D / dq, ec = E / dq;
+    const T ec2 = ec * ec;
+    const T linear = -(twice(dc) * T(k.lin));
+    const T quartic = ec2 - T(1.0);
+    const T quadratic = ((T(k.quad) * quartic) + T(1.0)) - (((dc * dc) * T(k.gm)) * T(k.gm));
+    const T eta = twice(dc) * T(k.gm);
+    const T quad2 = twice(quadratic), quart4 = fourfold(quartic), eta3 = (T(3.0) * eta) * quartic;
+    T x = T(1.0);
     int it = 0;
     bool conv = false;
     while (it < 1000) {
-        double f = ((((quartic * ((x * x) * x)) * (x - eta)) + (quadratic * (x * x))) + (linear * x)) + constant;
-        double fp = ((linear + ((2.0 * quadratic) * x)) + ((4.0 * quartic) * ((x * x) * x))) - (((3.0 * eta) * quartic) * (x * x));
-        double nx = x - (f / fp);
-        if (fabs(x - nx) < tol) { conv = true; break; }
+        const T x2 = x * x, x3 = x2 * x;
+        const T f = ((((quartic * x3) * (x - eta)) + (quadratic * x2)) + (linear * x)) + T(k.cst);
+        const T fp = ((linear + (quad2 * x)) + (quart4 * x3)) - (eta3 * x2);
+        const T nx = x - (f / fp);
+        if (nearer_zero(x - nx, tol)) { conv = true; break; }
         it += 1;
         x = nx;
+        if (hopeless(nx)) return C2P<T>{nx, nx, nx, nx, nx, nx, nx};
     }
-    if (!conv && capped) *capped = 1;
-    C2P r;
-    r.W = ((0.5 * ec) * x) * (1.0 + sqrt(1.0 + ((4.0 * ((g - 1.0) / g)) * ((1.0 - (dc * x)) / ((ec * ec) * (x * x))))));
-    r.h = 1.0 / (dc * x);
+    if (!conv && status) atomicOr(status, ST_NEWTON_CAP);
+    C2P<T> r;
+    const T dx = dc * x;
+    r.W = (half(ec) * x) * (T(1.0) + root(T(1.0) + (T(k.gm4) * ((T(1.0) - dx) / (ec2 * (x * x))))));
+    r.h = T(1.0) / dx;
     r.rho = D / r.W;
-    double rhw = (r.rho * r.h) * (r.W * r.W);
-    r.vx = Sx / rhw; r.vy = Sy / rhw; r.vz = Sz / rhw;
+    const T rhw = (r.rho * r.h) * (r.W * r.W);
+    const auto dr = divisor(rhw);
+    r.vx = Sx / dr; r.vy = Sy / dr; r.vz = Sz / dr;
     r.p = (rhw - D) - tau;
-    if (r.rho < 1e-8) r.rho = 1e-8;
-    if (r.p < 1e-8) r.p = 1e-8;
+    if (below(r.rho, 1e-8)) r.rho = T(1e-8);
+    if (below(r.p, 1e-8)) r.p = T(1e-8);
     return r;
 }
 
 // RelativisticEuler/RelativisticEulerEquationOfState.cpp:3-18
-CG_D double sr_enthalpy(double rho, double p, double g) { return 1.0 + ((p / rho) * (g / (g - 1.0))); }
-CG_D double sr_sound(double rho, double p, double g) {
-    double num = (g * p) / rho;
-    double den = 1.0 + ((p / rho) * (g / (g - 1.0)));
-    return sqrt(num / den);
+template <class T> CG_D T sr_enthalpy(T rho, T p, const GammaConst& k) { return T(1.0) + ((p / rho) * T(k.hg)); }
+template <class T> CG_D T sr_sound(T rho, T p, const GammaConst& k) {
+    const auto d = divisor(rho);
+    T num = (T(k.g) * p) / d;
+    T den = T(1.0) + ((p / d) * T(k.hg));
+    return root(num / den);
+}
+// 1 / sqrt(1 - v2), capped (RelativisticEuler/RelativisticEulerStateVector.cpp:116-136)
+template <class T> CG_D T lorentz(T v2) {
+    const bool fast = above(v2, 1.0 - 1e-8);
+    return T(1.0) / root(fast ? T(1.0 - 1e-8) : T(1.0) - v2);
 }
 
 // ============================================================== SR Euler (FP64)
 struct SRExact {
-    double g;
-    int* capped;  // optional: set when a Newton solve hits its cap
+    GammaConst k;
+    int* status;  // optional: gets ST_NEWTON_CAP when a Newton solve hits its cap
     static constexpr bool kCoords = false;
+    SRExact() = default;
+    explicit SRExact(double gamma, int* st = nullptr) : k(gamma), status(st) {}
     // RelativisticEuler/RelativisticEulerStateVector.cpp:116-136
-    CG_D void cons(const double* p, Pt, double* u) const {
-        double rho = p[0], vx = p[1], vy = p[2], vz = p[3], pr = p[4];
-        double v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
-        double W = 1.0 / sqrt(1.0 - v2);
-        if (v2 > 1.0 - 1e-8) W = 1.0 / sqrt(1.0 - 1e-8);
-        double h = sr_enthalpy(rho, pr, g);
-        double rhw = (rho * h) * (W * W);
+    template <class T> CG_D void cons(const T* p, Pt, T* u) const {
+        T rho = p[0], vx = p[1], vy = p[2], vz = p[3], pr = p[4];
+        T v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
+        T W = lorentz(v2);
+        T h = sr_enthalpy(rho, pr, k);
+        T rhw = (rho * h) * (W * W);
         u[0] = rho * W; u[1] = rhw * vx; u[2] = rhw * vy; u[3] = rhw * vz;
-        u[4] = (rhw - pr) - (rho * W);
+        u[4] = (rhw - pr) - u[0];
     }
-    CG_D void prim(const double* u, Pt, double* p) const {
-        C2P c = con2prim_exact(u[0], u[1], u[2], u[3], u[4], g, 1e-8, capped);
+    template <class T> CG_D void prim(const T* u, Pt, T* p) const {
+        C2P<T> c = con2prim_exact(V5<T>{{u[0], u[1], u[2], u[3], u[4]}}, k, 1e-8, status);
         p[0] = c.rho; p[1] = c.vx; p[2] = c.vy; p[3] = c.vz; p[4] = c.p;
     }
     // RelativisticEuler/RelativisticEulerStateVector.cpp:138-220 (x), :227-309 (y)
-    CG_D void flux(const double* u, int axis, Pt, double* f) const {
-        C2P c = con2prim_exact(u[0], u[1], u[2], u[3], u[4], g, 1e-8, capped);
-        double rhw = (c.rho * c.h) * (c.W * c.W);
-        double vn = axis == 0 ? c.vx : c.vy;
-        f[0] = (c.rho * c.W) * vn;
-        if (axis == 0) {
-            f[1] = (rhw * (c.vx * c.vx)) + c.p; f[2] = rhw * (c.vy * c.vx); f[3] = rhw * (c.vz * c.vx);
-        } else {
-            f[1] = rhw * (c.vx * c.vy); f[2] = (rhw * (c.vy * c.vy)) + c.p; f[3] = rhw * (c.vz * c.vy);
-        }
-        f[4] = (((rhw - c.p) - (c.rho * c.W)) * vn) + (c.p * vn);
+    template <class T> CG_D void flux(const T* u, int axis, Pt, T* f) const {
+        C2P<T> c = con2prim_exact(V5<T>{{u[0], u[1], u[2], u[3], u[4]}}, k, 1e-8, status);
+        T rhw = (c.rho * c.h) * (c.W * c.W);
+        T vn = axis == 0 ? c.vx : c.vy;
+        const T rw = c.rho * c.W;
+        f[0] = rw * vn;
+        const T nn = (rhw * (vn * vn)) + c.p, xy = rhw * (c.vx * c.vy);
+        f[1] = axis == 0 ? nn : xy;
+        f[2] = axis == 0 ? xy : nn;
+        f[3] = rhw * (c.vz * vn);
+        f[4] = (((rhw - c.p) - rw) * vn) + (c.p * vn);
     }
     // Solvers/RelativisticEulerSolvers.cpp:87-128 (2D: max(|vx|, |vy|) + c)
-    CG_D double wavespeed(const double* p, int dims, Pt) const {
-        double c = fabs(sr_sound(p[0], p[4], g));
-        if (dims == 1) return fabs(p[1]) + c;
-        return mx(fabs(p[1]), fabs(p[2])) + c;
+    template <class T> CG_D T wavespeed(const T* p, int dims, Pt) const {
+        T c = magnitude(sr_sound(p[0], p[4], k));
+        if (dims == 1) return magnitude(p[1]) + c;
+        return larger(magnitude(p[1]), magnitude(p[2])) + c;
     }
 };
 
 // ============================================================== Kerr-Schild spacetime (FP64)
 struct BHExact {
     double M, a, bx, by, bz;
-    // BlackHoleSpacetime.cpp:54-68
-    CG_D double radius(double dx, double dy, double dz) const {
-        double n2 = ((dx * dx) + (dy * dy)) + (dz * dz);
-        double ma2 = (M * M) * (a * a);
-        return sqrt(0.5 * ((n2 - ma2) + sqrt(((n2 - ma2) * (n2 - ma2)) + (4.0 * (ma2 * (dz * dz))))));
+    double ma2, am, horizon;  // M^2 a^2, a M, M (1 + sqrt(1 - a^2))
+    BHExact() = default;
+    BHExact(double mass, double spin, double x, double y, double z) : M(mass), a(spin), bx(x), by(y), bz(z) {
+        ma2 = (M * M) * (a * a);
+        am = a * M;
+        volatile double aa = a * a;  // rounded before the subtraction: host compilers may contract the two
+        horizon = M * (1.0 + ::sqrt(1.0 - aa));
     }
-    CG_D double H(double x, double y, double z) const {
-        double dx = x - bx, dy = y - by, dz = z - bz;
-        double r = radius(dx, dy, dz);
-        double ma2 = (M * M) * (a * a);
-        return -(M * ((r * r) * r)) / ((((r * r) * r) * r) + (ma2 * (dz * dz)));
+    // BlackHoleSpacetime.cpp:54-68
+    template <class T> CG_D T radius(T dx, T dy, T dz) const {
+        const T zz = dz * dz;
+        const T n2 = ((dx * dx) + (dy * dy)) + zz;
+        const T d = n2 - T(ma2);
+        return root(half(d + root((d * d) + fourfold(T(ma2) * zz))));
+    }
+    template <class T> CG_D T H(double x, double y, double z) const {
+        T dx = x - bx, dy = y - by, dz = z - bz;
+        T r = radius(dx, dy, dz);
+        const T r3 = (r * r) * r;
+        return -(T(M) * r3) / ((r3 * r) + (T(ma2) * (dz * dz)));
     }
     // BlackHoleSpacetime.cpp:70-90
-    CG_D void l(double x, double y, double z, double* o) const {
-        double dx = x - bx, dy = y - by, dz = z - bz;
-        double r = radius(dx, dy, dz);
-        double ma2 = (M * M) * (a * a);
-        o[0] = -((r * dx) + ((a * M) * dy)) / ((r * r) + ma2);
-        o[1] = -((r * dy) - ((a * M) * dx)) / ((r * r) + ma2);
+    template <class T> CG_D void l(double x, double y, double z, T* o) const {
+        T dx = x - bx, dy = y - by, dz = z - bz;
+        T r = radius(dx, dy, dz);
+        const auto d = divisor((r * r) + T(ma2));
+        o[0] = -((r * dx) + (T(am) * dy)) / d;
+        o[1] = -((r * dy) - (T(am) * dx)) / d;
         o[2] = -dz / r;
     }
     // H and l together (same arithmetic as the two separate calls)
-    CG_D void Hl(double x, double y, double z, double& h, double* o) const {
-        double dx = x - bx, dy = y - by, dz = z - bz;
-        double r = radius(dx, dy, dz);
-        double ma2 = (M * M) * (a * a);
-        h = -(M * ((r * r) * r)) / ((((r * r) * r) * r) + (ma2 * (dz * dz)));
-        o[0] = -((r * dx) + ((a * M) * dy)) / ((r * r) + ma2);
-        o[1] = -((r * dy) - ((a * M) * dx)) / ((r * r) + ma2);
+    template <class T> CG_D void Hl(double x, double y, double z, T& h, T* o) const {
+        T dx = x - bx, dy = y - by, dz = z - bz;
+        T r = radius(dx, dy, dz);
+        const T r2 = r * r, r3 = r2 * r;
+        h = -(T(M) * r3) / ((r3 * r) + (T(ma2) * (dz * dz)));
+        const auto d = divisor(r2 + T(ma2));
+        o[0] = -((r * dx) + (T(am) * dy)) / d;
+        o[1] = -((r * dy) - (T(am) * dx)) / d;
         o[2] = -dz / r;
     }
     // BlackHoleSpacetime.cpp:92-113 with "r + (y - y_BH)" of :108 as written
-    CG_D void L4(double x, double y, double z, double* o) const {
-        double dx = x - bx, dy = y - by, dz = z - bz;
-        double r = radius(dx, dy, dz);
-        double ma2 = (M * M) * (a * a);
-        o[0] = -1.0;
-        o[1] = -((r * dx) + ((a * M) * dy)) / ((r * r) + ma2);
-        o[2] = -((r + dy) - ((a * M) * dx)) / ((r * r) + ma2);
+    template <class T> CG_D void L4(double x, double y, double z, T* o) const {
+        T dx = x - bx, dy = y - by, dz = z - bz;
+        T r = radius(dx, dy, dz);
+        const auto d = divisor((r * r) + T(ma2));
+        o[0] = T(-1.0);
+        o[1] = -((r * dx) + (T(am) * dy)) / d;
+        o[2] = -((r + dy) - (T(am) * dx)) / d;
         o[3] = -dz / r;
     }
     // BlackHoleSpacetime.cpp:153-186
-    CG_D void gamma(double x, double y, double z, double* m) const {
-        double h, v[3];
+    template <class T> CG_D void gamma(double x, double y, double z, T* m) const {
+        T h, v[3];
         Hl(x, y, z, h, v);
+        gamma_of(h, v, m);
+    }
+    template <class T> CG_D void gamma_of(T h, const T* v, T* m) const {
+        const T h2 = twice(h);
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) m[3 * i + j] = (i == j ? 1.0 : 0.0) - (((2.0 * h) * v[i]) * v[j]);
+            for (int j = 0; j < 3; j++) m[3 * i + j] = T(i == j ? 1.0 : 0.0) - ((h2 * v[i]) * v[j]);
     }
     // BlackHoleSpacetime.cpp:188-228
-    CG_D void g4(double x, double y, double z, double* m) const {
-        double h = H(x, y, z), v[4];
+    template <class T> CG_D void g4(double x, double y, double z, T* m) const {
+        T h = H<T>(x, y, z), v[4];
         L4(x, y, z, v);
+        const T h2 = twice(h);
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                double eta = (i == j) ? ((i == 0) ? -1.0 : 1.0) : 0.0;
-                m[4 * i + j] = eta - (((2.0 * h) * v[i]) * v[j]);
+                const double eta = (i == j) ? ((i == 0) ? -1.0 : 1.0) : 0.0;
+                m[4 * i + j] = T(eta) - ((h2 * v[i]) * v[j]);
             }
     }
-    CG_D double lapse(double x, double y, double z) const { return 1.0 / sqrt(1.0 - (2.0 * H(x, y, z))); }
-    CG_D void shiftv(double x, double y, double z, double* b) const {
-        double h, v[3];
+    // lapse and shift from one H/l evaluation
+    template <class T> CG_D void lapse_shift(double x, double y, double z, T& al, T* b) const {
+        T h, v[3];
         Hl(x, y, z, h, v);
-#pragma unroll
-        for (int i = 0; i < 3; i++) b[i] = ((2.0 * h) / (1.0 - (2.0 * h))) * v[i];
+        lapse_shift_of(h, v, al, b);
     }
-    // lapse and shift from one H/l evaluation (same arithmetic as the separate calls)
-    CG_D void lapse_shift(double x, double y, double z, double& al, double* b) const {
-        double h, v[3];
-        Hl(x, y, z, h, v);
-        al = 1.0 / sqrt(1.0 - (2.0 * h));
+    template <class T> CG_D void lapse_shift_of(T h, const T* v, T& al, T* b) const {
+        const T h2 = twice(h), d = T(1.0) - h2;
+        al = T(1.0) / root(d);
+        const T f = h2 / d;
 #pragma unroll
-        for (int i = 0; i < 3; i++) b[i] = ((2.0 * h) / (1.0 - (2.0 * h))) * v[i];
+        for (int i = 0; i < 3; i++) b[i] = f * v[i];
     }
     // BlackHoleSpacetime.cpp:372-386
     CG_D bool excised(double x, double y, double z) const {
-        double r = sqrt((((x - bx) * (x - bx)) + ((y - by) * (y - by))) + ((z - bz) * (z - bz)));
-        return r <= (M * (1.0 + sqrt(1.0 - (a * a))));
+        const xd dx = x - bx, dy = y - by, dz = z - bz;
+        double r = root(((dx * dx) + (dy * dy)) + (dz * dz)).v;
+        if (!xm::finite(r)) r = ::sqrt((((x - bx) * (x - bx)) + ((y - by) * (y - by))) + ((z - bz) * (z - bz)));
+        return r <= horizon;
     }
 };
 
 // Mathematics/MatrixAlgebra.cpp:106-149: cofactor expansion along row 0 down to 2x2.
-CG_D double det2(double a00, double a01, double a10, double a11) { return (a00 * a11) - (a10 * a01); }
-CG_D double det3(const double* m) {
-    double d = 0.0;
+template <class T> CG_D T det2(T a00, T a01, T a10, T a11) { return (a00 * a11) - (a10 * a01); }
+template <class T> CG_D T det3(const T* m) {
+    T d = T(0.0);
     d = d + (m[0] * det2(m[4], m[5], m[7], m[8]));
     d = d - (m[1] * det2(m[3], m[5], m[6], m[8]));
     d = d + (m[2] * det2(m[3], m[4], m[6], m[7]));
     return d;
 }
-CG_D double det4(const double* m) {
-    double d = 0.0;
-#pragma unroll
+// (the 4x4 algebra keeps its outer loops: it runs once per cell and step, and unrolled it is thousands
+// of instructions)
+template <class T> CG_D T det4(const T* m) {
+    T d = T(0.0);
+#pragma unroll 1
     for (int i = 0; i < 4; i++) {
-        double c[9];
+        T c[9];
 #pragma unroll
         for (int j = 0; j < 3; j++)
 #pragma unroll
@@ -292,370 +380,532 @@ CG_D double det4(const double* m) {
     }
     return d;
 }
-template <int N> CG_D void matmul_n(const double* a, const double* b, double* c) {
-#pragma unroll
+template <int N, class T> CG_D void matmul_n(const T* a, const T* b, T* c) {
+#pragma unroll N < 4 ? N : 1
     for (int i = 0; i < N; i++)
 #pragma unroll
         for (int j = 0; j < N; j++) {
-            double s = 0.0;
+            T s = T(0.0);
 #pragma unroll
             for (int k = 0; k < N; k++) s = s + (a[N * i + k] * b[N * k + j]);
             c[N * i + j] = s;
         }
 }
-template <int N> CG_D double trace_n(const double* m) {
-    double t = 0.0;
+template <int N, class T> CG_D T trace_n(const T* m) {
+    T t = T(0.0);
 #pragma unroll
     for (int i = 0; i < N; i++) t = t + m[N * i + i];
     return t;
 }
 // Mathematics/MatrixAlgebra.cpp:151-194 (Cayley-Hamilton)
-CG_D void inverse3(const double* m, double* o) {
-    double d = det3(m), tr = trace_n<3>(m), m2[9];
+template <class T> CG_D void inverse3(const T* m, T* o) {
+    T d = det3(m), tr = trace_n<3>(m), m2[9];
     matmul_n<3>(m, m, m2);
-    double tr2 = trace_n<3>(m2);
-    double s = 0.5 * ((tr * tr) - tr2);
-    double inv = 1.0 / d;
+    T tr2 = trace_n<3>(m2);
+    T s = half((tr * tr) - tr2);
+    T inv = T(1.0) / d;
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
-        for (int j = 0; j < 3; j++) o[3 * i + j] = inv * (((s * (i == j ? 1.0 : 0.0)) - (tr * m[3 * i + j])) + m2[3 * i + j]);
+        for (int j = 0; j < 3; j++) o[3 * i + j] = inv * (((i == j ? s : times_zero(s)) - (tr * m[3 * i + j])) + m2[3 * i + j]);
 }
-CG_D void inverse4(const double* m, double* o) {
-    double d = det4(m), tr = trace_n<4>(m), m2[16], m3[16];
+template <class T> CG_D void inverse4(const T* m, T* o) {
+    T d = det4(m), tr = trace_n<4>(m), m2[16], m3[16];
     matmul_n<4>(m, m, m2);
     matmul_n<4>(m2, m, m3);
-    double tr2 = trace_n<4>(m2), tr3 = trace_n<4>(m3);
-    double c0 = (1.0 / 6.0) * ((((tr * tr) * tr) - ((3.0 * tr) * tr2)) + (2.0 * tr3));
-    double c1 = 0.5 * ((tr * tr) - tr2);
-    double inv = 1.0 / d;
-#pragma unroll
+    T tr2 = trace_n<4>(m2), tr3 = trace_n<4>(m3);
+    T c0 = T(1.0 / 6.0) * ((((tr * tr) * tr) - ((T(3.0) * tr) * tr2)) + twice(tr3));
+    T c1 = half((tr * tr) - tr2);
+    T inv = T(1.0) / d;
+#pragma unroll 1
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            o[4 * i + j] = inv * ((((c0 * (i == j ? 1.0 : 0.0)) - (c1 * m[4 * i + j])) + (tr * m2[4 * i + j])) - m3[4 * i + j]);
+            o[4 * i + j] = inv * ((((i == j ? c0 : times_zero(c0)) - (c1 * m[4 * i + j])) + (tr * m2[4 * i + j])) - m3[4 * i + j]);
 }
 
 // ============================================================== GR Euler (FP64)
+// The metric at one point, as the state functions take it: spatial metric, sqrt(det gamma), lapse, shift.
+template <class T> struct Metric { T gm[9], sg, al, be[3]; };
+// What the source term takes beyond it: inverse 4-metric, centred derivatives of the lapse, shift and
+// spatial metric, extrinsic curvature.
+template <class T> struct SourceMetric { T gi[16], da[3], db[9], dgm[27], K[9]; };
+
 struct GRExact {
-    double g;
+    GammaConst k;
     BHExact bh;
-    double h;      // finite-difference spacing of the metric derivatives (the cell spacing)
-    int* capped;
+    double h, ih, hs;  // finite-difference spacing of the metric derivatives (the cell spacing), 1 / h, h / 2
+    int* status;       // as in SRExact
     static constexpr bool kCoords = true;
+    GRExact() = default;
+    GRExact(double gamma, const double* hole, double spacing, int* st = nullptr)
+        : k(gamma), bh(hole[0], hole[1], hole[2], hole[3], hole[4]), h(spacing), ih(1.0 / spacing), hs(0.5 * spacing),
+          status(st) {}
 
-    CG_D double detg(Pt p) const { double m[9]; bh.gamma(p.x, p.y, p.z, m); return det3(m); }
-
-    // BlackHoleEuler/BlackHoleEulerStateVector.cpp:118-157 (energy with W, not W^2, at :154)
-    CG_D void cons(const double* p, Pt q, double* u) const {
-        double m[9];
-        bh.gamma(q.x, q.y, q.z, m);
-        double dg = det3(m);
-        double v[3] = {p[1], p[2], p[3]};
-        double v2 = 0.0;
+    template <class T> CG_D void metric(Pt q, Metric<T>& o) const {
+        T hh, l[3];
+        bh.Hl(q.x, q.y, q.z, hh, l);
+        bh.gamma_of(hh, l, o.gm);
+        o.sg = root(det3(o.gm));
+        bh.lapse_shift_of(hh, l, o.al, o.be);
+    }
+    // gamma_ij v^i v^j in the reference's order
+    template <class T> CG_D T square(const T* m, const T* v) const {
+        T v2 = T(0.0);
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
             for (int j = 0; j < 3; j++) v2 = v2 + ((m[3 * i + j] * v[i]) * v[j]);
-        double W = 1.0 / sqrt(1.0 - v2);
-        if (v2 > 1.0 - 1e-8) W = 1.0 / sqrt(1.0 - 1e-8);
-        double hh = sr_enthalpy(p[0], p[4], g);
-        double sg = sqrt(dg);
-        u[0] = (sg * p[0]) * W;
-#pragma unroll
-        for (int k = 0; k < 3; k++) u[1 + k] = (((sg * p[0]) * hh) * (W * W)) * v[k];
-        u[4] = sg * ((((p[0] * hh) * W) - p[4]) - (p[0] * W));
+        return v2;
     }
-    CG_D C2P c2p(const double* u, double sg, double tol) const {
-        return con2prim_exact(u[0] / sg, u[1] / sg, u[2] / sg, u[3] / sg, u[4] / sg, g, tol, capped);
+    // BlackHoleEuler/BlackHoleEulerStateVector.cpp:118-157 (energy with W, not W^2, at :154)
+    template <class T> CG_D void cons_in(const Metric<T>& g, const T* p, T* u) const {
+        const T W = lorentz(square(g.gm, p + 1));
+        const T hh = sr_enthalpy(p[0], p[4], k);
+        const T sr = g.sg * p[0];
+        u[0] = sr * W;
+        const T srhw = (sr * hh) * (W * W);
+#pragma unroll
+        for (int f = 0; f < 3; f++) u[1 + f] = srhw * p[1 + f];
+        u[4] = g.sg * ((((p[0] * hh) * W) - p[4]) - (p[0] * W));
+    }
+    template <class T> CG_D C2P<T> c2p(const T* u, T sg, double tol) const {
+        const auto d = divisor(sg);
+        return con2prim_exact(V5<T>{{u[0] / d, u[1] / d, u[2] / d, u[3] / d, u[4] / d}}, k, tol, status);
     }
     // BlackHoleEuler/BlackHoleEulerStateVector.cpp:30-103
-    CG_D void prim(const double* u, Pt q, double* p) const {
-        C2P c = c2p(u, sqrt(detg(q)), 1e-8);
+    template <class T> CG_D void prim_in(const Metric<T>& g, const T* u, T* p) const {
+        C2P<T> c = c2p(u, g.sg, 1e-8);
         p[0] = c.rho; p[1] = c.vx; p[2] = c.vy; p[3] = c.vz; p[4] = c.p;
     }
     // BlackHoleEuler/BlackHoleEulerStateVector.cpp:159-250 (x, tol 1e-10) and :259-350 (y)
-    CG_D void flux(const double* u, int axis, Pt q, double* f) const {
-        double sg = sqrt(detg(q));
-        double al, be[3];
-        bh.lapse_shift(q.x, q.y, q.z, al, be);
-        C2P c = c2p(u, sg, axis == 0 ? 1e-10 : 1e-8);
-        double as = al * sg;
-        double rhw = (c.rho * c.h) * (c.W * c.W);
-        double vn = axis == 0 ? c.vx : c.vy;
-        double w = vn - ((axis == 0 ? be[0] : be[1]) / al);
-        f[0] = as * ((c.rho * c.W) * w);
-        if (axis == 0) {
-            f[1] = as * ((rhw * (c.vx * w)) + c.p);
-            f[2] = as * (rhw * (c.vy * w));
-        } else {
-            f[1] = as * (rhw * (c.vx * w));
-            f[2] = as * ((rhw * (c.vy * w)) + c.p);
-        }
+    template <class T> CG_D void flux_in(const Metric<T>& g, const T* u, int axis, T* f) const {
+        C2P<T> c = c2p(u, g.sg, axis == 0 ? 1e-10 : 1e-8);
+        const T as = g.al * g.sg;
+        const T rhw = (c.rho * c.h) * (c.W * c.W);
+        const T vn = axis == 0 ? c.vx : c.vy;
+        const T w = vn - ((axis == 0 ? g.be[0] : g.be[1]) / g.al);
+        const T rw = c.rho * c.W;
+        f[0] = as * (rw * w);
+        const T x = rhw * (c.vx * w), y = rhw * (c.vy * w);
+        f[1] = as * (axis == 0 ? x + c.p : x);
+        f[2] = as * (axis == 0 ? y : y + c.p);
         f[3] = as * (rhw * (c.vz * w));
-        f[4] = as * ((((rhw - c.p) - (c.rho * c.W)) * w) + (c.p * vn));
+        f[4] = as * ((((rhw - c.p) - rw) * w) + (c.p * vn));
     }
     // ---- metric derivatives (BlackHoleSpacetime.cpp:115-151, :250-334), centred with spacing h
     CG_D Pt off(Pt q, int d, double s) const {
         if (d == 0) q.x = q.x + s; else if (d == 1) q.y = q.y + s; else q.z = q.z + s;
         return q;
     }
-    // BlackHoleSpacetime.cpp:336-370
-    CG_D void Kij(Pt q, double al, double* K) const {
-        double Hs, v[3];
-        bh.Hl(q.x, q.y, q.z, Hs, v);
-        double dh[3], dv[9];
-        const double hs = 0.5 * h;
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            Pt p1 = off(q, d, hs), p0 = off(q, d, -hs);
-            double h1, h0, a1[3], a0[3];
-            bh.Hl(p1.x, p1.y, p1.z, h1, a1);
-            bh.Hl(p0.x, p0.y, p0.z, h0, a0);
-            dh[d] = (h1 - h0) / h;
-#pragma unroll
-            for (int c = 0; c < 3; c++) dv[3 * d + c] = (1.0 / h) * (a1[c] - a0[c]);
-        }
-#pragma unroll
+    // BlackHoleSpacetime.cpp:336-370 from H, l at the point (Hs, v) and its centred differences
+    template <class T> CG_D void Kij_of(T al, T Hs, const T* v, const T* dh, const T* dv, T* K) const {
+        const T al2 = twice(al), a2hh = al2 * (Hs * Hs), a2h = al2 * Hs;
+#pragma unroll 1
         for (int i = 0; i < 3; i++)
-#pragma unroll
+#pragma unroll 1
             for (int j = 0; j < 3; j++) {
-                double k = al * ((((-(v[i] * dh[j])) - (v[j] * dh[i])) - (Hs * dv[3 * j + i])) - (Hs * dv[3 * i + j]));
+                T kk = al * (((-(v[i] * dh[j]) - (v[j] * dh[i])) - (Hs * dv[3 * j + i])) - (Hs * dv[3 * i + j]));
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
-                    k = k + (((al * 2.0) * (Hs * Hs)) * (((v[i] * v[c]) * dv[3 * c + j]) + ((v[j] * v[c]) * dv[3 * c + i])));
-                    k = k + ((((((al * 2.0) * Hs) * v[i]) * v[j]) * v[c]) * dh[c]);
+                    kk = kk + (a2hh * (((v[i] * v[c]) * dv[3 * c + j]) + ((v[j] * v[c]) * dv[3 * c + i])));
+                    kk = kk + ((((a2h * v[i]) * v[j]) * v[c]) * dh[c]);
                 }
-                K[3 * i + j] = k;
+                K[3 * i + j] = kk;
             }
     }
     // The metric part of the source term at q: inverse 4-metric, centred derivatives of the lapse,
     // shift and spatial metric (spacing h), extrinsic curvature (BlackHoleSpacetime.cpp:115-151,
-    // :230-370).
-    CG_D void source_metric(Pt q, double al, double* gi, double* da, double* db, double* dgm, double* K) const {
-        double g4m[16];
+    // :230-370).  H and l are evaluated once per point; every quantity there comes from them.
+    template <class T> CG_D void source_metric(Pt q, T al, T* gi, T* da, T* db, T* dgm, T* K) const {
+        T g4m[16];
         bh.g4(q.x, q.y, q.z, g4m);
         inverse4(g4m, gi);
-        const double hs = 0.5 * h;
-#pragma unroll
+        const auto dh_ = divisor(T(h));
+        T dH[3], dl[9], Hs, v[3];
+#pragma unroll 1
         for (int d = 0; d < 3; d++) {
             Pt p1 = off(q, d, hs), p0 = off(q, d, -hs);
-            double a1, a0, b1[3], b0[3], g1[9], g0[9];
-            bh.lapse_shift(p1.x, p1.y, p1.z, a1, b1);
-            bh.lapse_shift(p0.x, p0.y, p0.z, a0, b0);
-            bh.gamma(p1.x, p1.y, p1.z, g1);
-            bh.gamma(p0.x, p0.y, p0.z, g0);
-            da[d] = (a1 - a0) / h;
+            T h1, h0, l1[3], l0[3], a1, a0, b1[3], b0[3], g1[9], g0[9];
+            bh.Hl(p1.x, p1.y, p1.z, h1, l1);
+            bh.Hl(p0.x, p0.y, p0.z, h0, l0);
+            bh.lapse_shift_of(h1, l1, a1, b1);
+            bh.lapse_shift_of(h0, l0, a0, b0);
+            bh.gamma_of(h1, l1, g1);
+            bh.gamma_of(h0, l0, g0);
+            da[d] = (a1 - a0) / dh_;
+            dH[d] = (h1 - h0) / dh_;
 #pragma unroll
-            for (int k = 0; k < 3; k++) db[3 * d + k] = (1.0 / h) * (b1[k] - b0[k]);
+            for (int c = 0; c < 3; c++) db[3 * d + c] = T(ih) * (b1[c] - b0[c]);
 #pragma unroll
-            for (int k = 0; k < 9; k++) dgm[9 * d + k] = (1.0 / h) * (g1[k] - g0[k]);
+            for (int c = 0; c < 3; c++) dl[3 * d + c] = T(ih) * (l1[c] - l0[c]);
+#pragma unroll
+            for (int c = 0; c < 9; c++) dgm[9 * d + c] = T(ih) * (g1[c] - g0[c]);
         }
-        Kij(q, al, K);
+        bh.Hl(q.x, q.y, q.z, Hs, v);
+        Kij_of(al, Hs, v, dH, dl, K);
     }
     // BlackHoleEuler/BlackHoleEulerStateVector.cpp:359-510
-    CG_D void source(const double* u, Pt q, double* s) const {
-        double gm[9];
-        bh.gamma(q.x, q.y, q.z, gm);
-        double dg = det3(gm);
-        double al, be[3];
-        bh.lapse_shift(q.x, q.y, q.z, al, be);
-        C2P c = c2p(u, sqrt(dg), 1e-8);
-        double gi[16], da[3], db[9], dgm[27], K[9];
-        source_metric(q, al, gi, da, db, dgm, K);
-        double uu[4];
+    template <class T> CG_D void source_in(const Metric<T>& g, const SourceMetric<T>& sm, const T* u, T* s) const {
+        C2P<T> c = c2p(u, g.sg, 1e-8);
+        const T al = g.al, sg = g.sg;
+        const T *be = g.be, *gm = g.gm, *gi = sm.gi, *da = sm.da, *db = sm.db, *dgm = sm.dgm, *K = sm.K;
+        T uu[4];
         uu[0] = c.W / al;
-        uu[1] = ((al * uu[0]) * c.vx) - (be[0] * uu[0]);
-        uu[2] = ((al * uu[0]) * c.vy) - (be[1] * uu[0]);
-        uu[3] = ((al * uu[0]) * c.vz) - (be[2] * uu[0]);
-        double T[16];
-#pragma unroll
+        const T au = al * uu[0];
+        uu[1] = (au * c.vx) - (be[0] * uu[0]);
+        uu[2] = (au * c.vy) - (be[1] * uu[0]);
+        uu[3] = (au * c.vz) - (be[2] * uu[0]);
+        T E[16];
+        const T rh = c.rho * c.h;
+#pragma unroll 1
         for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) T[4 * i + j] = (((c.rho * c.h) * uu[i]) * uu[j]) + (c.p * gi[4 * i + j]);
-        double S[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        double vc[3];
+#pragma unroll 1
+            for (int j = 0; j < 4; j++) E[4 * i + j] = ((rh * uu[i]) * uu[j]) + (c.p * gi[4 * i + j]);
+        T S[5] = {T(0.0), T(0.0), T(0.0), T(0.0), T(0.0)};
+        T vc[3];
 #pragma unroll
         for (int i = 0; i < 3; i++) vc[i] = ((gm[3 * i + 0] * c.vx) + (gm[3 * i + 1] * c.vy)) + (gm[3 * i + 2] * c.vz);
-        double rhw = (c.rho * c.h) * (c.W * c.W);
-#pragma unroll
+        const T rhw = rh * (c.W * c.W);
+#pragma unroll 1
         for (int i = 0; i < 3; i++) {
-#pragma unroll
+#pragma unroll 1
             for (int j = 0; j < 3; j++) {
+                const T hb = half(be[j]);
 #pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    double dgijk = dgm[9 * i + 3 * j + k];
-                    S[i + 1] = S[i + 1] + (T[0] * (((0.5 * be[j]) * be[k]) * dgijk));
-                    S[i + 1] = S[i + 1] + ((T[j + 1] * be[k]) * dgijk);
-                    S[i + 1] = S[i + 1] + (0.5 * (T[4 * (j + 1) + (k + 1)] * dgijk));
+                for (int m = 0; m < 3; m++) {
+                    const T dgijk = dgm[9 * i + 3 * j + m];
+                    S[i + 1] = S[i + 1] + (E[0] * ((hb * be[m]) * dgijk));
+                    S[i + 1] = S[i + 1] + ((E[j + 1] * be[m]) * dgijk);
+                    S[i + 1] = S[i + 1] + half(E[4 * (j + 1) + (m + 1)] * dgijk);
                 }
                 S[i + 1] = S[i + 1] + (((rhw * vc[j]) / al) * db[3 * i + j]);
             }
-            S[i + 1] = S[i + 1] - ((T[0] * al) * da[i]);
+            S[i + 1] = S[i + 1] - ((E[0] * al) * da[i]);
         }
-#pragma unroll
+#pragma unroll 1
         for (int i = 0; i < 3; i++) {
-#pragma unroll
+#pragma unroll 1
             for (int j = 0; j < 3; j++) {
-                S[4] = S[4] + (T[0] * ((be[i] * be[j]) * K[3 * i + j]));
-                S[4] = S[4] + (T[i + 1] * ((2.0 * be[j]) * K[3 * i + j]));
-                S[4] = S[4] + (T[4 * (i + 1) + (j + 1)] * K[3 * i + j]);
+                S[4] = S[4] + (E[0] * ((be[i] * be[j]) * K[3 * i + j]));
+                S[4] = S[4] + (E[i + 1] * (twice(be[j]) * K[3 * i + j]));
+                S[4] = S[4] + (E[4 * (i + 1) + (j + 1)] * K[3 * i + j]);
             }
-            S[4] = S[4] - (T[0] * (be[i] * da[i]));
-            S[4] = S[4] - (T[i + 1] * da[i]);
+            S[4] = S[4] - (E[0] * (be[i] * da[i]));
+            S[4] = S[4] - (E[i + 1] * da[i]);
         }
-        double f = al * sqrt(dg);
+        const T f = al * sg;
 #pragma unroll
-        for (int k = 0; k < 5; k++) s[k] = f * S[k];
+        for (int i = 0; i < 5; i++) s[i] = f * S[i];
     }
     // BlackHoleEuler/BlackHoleEulerStateVector.cpp:519-549, eigenvalues
     // BlackHoleEuler/BlackHoleEulerEigenvalues.cpp:3-96 (largest signed eigenvalue)
-    CG_D double sound_speed(const double* p, Pt q) const {
-        double al, be[3];
-        bh.lapse_shift(q.x, q.y, q.z, al, be);
-        double gm[9], gs[9];
-        bh.gamma(q.x, q.y, q.z, gm);
+    template <class T> CG_D T sound_speed(const T* p, Pt q) const {
+        T hh, l[3], al, be[3], gm[9], gs[9];
+        bh.Hl(q.x, q.y, q.z, hh, l);
+        bh.lapse_shift_of(hh, l, al, be);
+        bh.gamma_of(hh, l, gm);
         inverse3(gm, gs);
-        double cs = sr_sound(p[0], p[4], g);
-        double v[3] = {p[1], p[2], p[3]};
-        double v2 = 0.0;
-#pragma unroll
-        for (int i = 0; i < 3; i++)
-#pragma unroll
-            for (int j = 0; j < 3; j++) v2 = v2 + ((gm[3 * i + j] * v[i]) * v[j]);
-        double s = 0.0;
+        const T cs = sr_sound(p[0], p[4], k), c2 = cs * cs;
+        const T* v = p + 1;
+        const T v2 = square(gm, v);
+        const T o1 = T(1.0) - (v2 * c2), o2 = T(1.0) - c2, o3 = T(1.0) - v2;
+        const T pre = al / o1;
+        T s = T(0.0);
 #pragma unroll
         for (int i = 0; i < 3; i++) {
-            double mat = (al * v[i]) - be[i];
-            double rt = sqrt((1.0 - v2) * ((gs[3 * i + i] * (1.0 - (v2 * (cs * cs)))) - ((v[i] * v[i]) * (1.0 - (cs * cs)))));
-            double pre = al / (1.0 - (v2 * (cs * cs)));
-            double fast = (pre * ((v[i] * (1.0 - (cs * cs))) + (cs * rt))) - be[i];
-            double slow = (pre * ((v[i] * (1.0 - (cs * cs))) - (cs * rt))) - be[i];
-            if (mat > s) s = mat;
-            if (fast > s) s = fast;
-            if (slow > s) s = slow;
+            const T mat = (al * v[i]) - be[i];
+            const T rt = root(o3 * ((gs[3 * i + i] * o1) - ((v[i] * v[i]) * o2)));
+            const T fast = (pre * ((v[i] * o2) + (cs * rt))) - be[i];
+            const T slow = (pre * ((v[i] * o2) - (cs * rt))) - be[i];
+            // not finite here: every eigenvalue must show in the result (a comparison would drop it)
+            if (hopeless(mat) || hopeless(fast) || hopeless(slow)) return fast + slow + mat;
+            if (exceeds(mat, s)) s = mat;
+            if (exceeds(fast, s)) s = fast;
+            if (exceeds(slow, s)) s = slow;
         }
         return s;
     }
+    // the state functions at a point (state-level and per-interface calls)
+    template <class T> CG_D void cons(const T* p, Pt q, T* u) const;
+    template <class T> CG_D void prim(const T* u, Pt q, T* p) const;
+    template <class T> CG_D void flux(const T* u, int axis, Pt q, T* f) const;
+    template <class T> CG_D void source(const T* u, Pt q, T* s) const;
 };
+
+// One copy per number type: the functions are thousands of cycles long and used at many places.  S is a
+// kernel's parameter (__grid_constant__) or the copy of it that a slow path holds; the metrics lie in local
+// memory, formed once per point and shared by every state converted there.
+template <class T> __device__ __noinline__ void gr_metric(const GRExact* S, Pt q, Metric<T>* o) { S->metric(q, *o); }
+template <class T> __device__ __noinline__ V5<T> gr_cons(const GRExact* S, const Metric<T>* g, V5<T> p) {
+    V5<T> o;
+    S->cons_in(*g, p.v, o.v);
+    return o;
+}
+template <class T> __device__ __noinline__ V5<T> gr_prim(const GRExact* S, const Metric<T>* g, V5<T> u) {
+    V5<T> o;
+    S->prim_in(*g, u.v, o.v);
+    return o;
+}
+template <class T> __device__ __noinline__ V5<T> gr_flux(const GRExact* S, const Metric<T>* g, V5<T> u, int axis) {
+    V5<T> o;
+    S->flux_in(*g, u.v, axis, o.v);
+    return o;
+}
+template <class T> __device__ __noinline__ void gr_source_metric(const GRExact* S, Pt q, T al, SourceMetric<T>* o) {
+    S->source_metric(q, al, o->gi, o->da, o->db, o->dgm, o->K);
+}
+template <class T>
+__device__ __noinline__ V5<T> gr_source(const GRExact* S, const Metric<T>* g, const SourceMetric<T>* sm, V5<T> u) {
+    V5<T> o;
+    S->source_in(*g, *sm, u.v, o.v);
+    return o;
+}
+template <class T> CG_D V5<T> five(const T* a) { return V5<T>{{a[0], a[1], a[2], a[3], a[4]}}; }
+template <class T> CG_D void give(const V5<T>& a, T* o) {
+#pragma unroll
+    for (int k = 0; k < 5; k++) o[k] = a.v[k];
+}
+template <class T> CG_D void GRExact::cons(const T* p, Pt q, T* u) const {
+    Metric<T> g;
+    gr_metric(this, q, &g);
+    give(gr_cons(this, &g, five(p)), u);
+}
+template <class T> CG_D void GRExact::prim(const T* u, Pt q, T* p) const {
+    Metric<T> g;
+    gr_metric(this, q, &g);
+    give(gr_prim(this, &g, five(u)), p);
+}
+template <class T> CG_D void GRExact::flux(const T* u, int axis, Pt q, T* f) const {
+    Metric<T> g;
+    gr_metric(this, q, &g);
+    give(gr_flux(this, &g, five(u), axis), f);
+}
+template <class T> CG_D void GRExact::source(const T* u, Pt q, T* s) const {
+    Metric<T> g;
+    SourceMetric<T> sm;
+    gr_metric(this, q, &g);
+    gr_source_metric(this, q, g.al, &sm);
+    give(gr_source(this, &g, &sm, five(u)), s);
+}
 
 // ============================================================== generic evolution pieces
 // Half-step evolution (Solvers/EulerSolvers.cpp:174-223; SR Solvers/RelativisticEulerSolvers.cpp:148-199;
-// GR Solvers/BlackHoleEulerSolvers.cpp:234-307).  Produces the left- and/or right-face state as
-// primitives (the reference's evolved EulerStateVector).
+// GR Solvers/BlackHoleEulerSolvers.cpp:234-307) from the conserved states of the cell and its two
+// neighbours.  Produces the left- and/or right-face state as primitives (the reference's evolved
+// EulerStateVector).
 template <class Sys, class T>
-CG_D void evolve_half_exact(const Sys& S, const T* l, const T* m, const T* r, Pt xc, int axis, double dx, double dt,
-                            T w, int lim, T* left_face, T* right_face) {
-    T ul[5], um[5], ur[5], sl[5];
-    S.cons(l, shift_pt(xc, axis, -dx), ul);
-    S.cons(m, xc, um);
-    S.cons(r, shift_pt(xc, axis, dx), ur);
-    slope_exact(ul, um, ur, w, lim, sl);
+CG_D void evolve_half_cons(const Sys& S, const T* ul, const T* um, const T* ur, Pt xc, int axis, double dx,
+                           const StepRatio& st, const Bias& w, int lim, T* left_face, T* right_face) {
     T UL[5], UR[5], FL[5], FR[5];
 #pragma unroll
-    for (int k = 0; k < 5; k++) { UL[k] = um[k] - (T(0.5) * sl[k]); UR[k] = um[k] + (T(0.5) * sl[k]); }
+    for (int k = 0; k < 5; k++) {
+        const T hs = half(limited_slope(um[k] - ul[k], ur[k] - um[k], w, lim));
+        UL[k] = um[k] - hs;
+        UR[k] = um[k] + hs;
+    }
     S.flux(UL, axis, shift_pt(xc, axis, -(dx * 0.5)), FL);
     S.flux(UR, axis, shift_pt(xc, axis, dx * 0.5), FR);
-    const T s = T(0.5) * (T(dt) / T(dx));
-    T a[5], b[5];
+    const T s = half(T(st.d));
 #pragma unroll
     for (int k = 0; k < 5; k++) {
         T ev = s * (FL[k] - FR[k]);
-        a[k] = UL[k] + ev;
-        b[k] = UR[k] + ev;
+        UL[k] = UL[k] + ev;
+        UR[k] = UR[k] + ev;
     }
-    if (left_face) S.prim(a, shift_pt(xc, axis, -(dx * 0.5)), left_face);
-    if (right_face) S.prim(b, shift_pt(xc, axis, dx * 0.5), right_face);
+    if (left_face) S.prim(UL, shift_pt(xc, axis, -(dx * 0.5)), left_face);
+    if (right_face) S.prim(UR, shift_pt(xc, axis, dx * 0.5), right_face);
 }
-
-// FORCE flux of two primitive states at interface xf (Solvers/EulerFirstOrderSolver.cpp:3-59;
-// GR Solvers/BlackHoleEulerFirstOrderSolver.cpp:3-47).
+// ... from their primitive states
 template <class Sys, class T>
-CG_D void force_exact(const Sys& S, const T* L, const T* R, Pt xf, int axis, double dx, double dt, T* F) {
-    T uL[5], uR[5], fL[5], fR[5], us[5], fs[5];
-    Pt pl = shift_pt(xf, axis, -(dx * 0.5)), pr = shift_pt(xf, axis, dx * 0.5);
-    S.cons(L, pl, uL);
-    S.cons(R, pr, uR);
-    S.flux(uL, axis, pl, fL);
-    S.flux(uR, axis, pr, fR);
-    const T c = T(dx) / T(dt), d = T(dt) / T(dx);
-#pragma unroll
-    for (int k = 0; k < 5; k++) us[k] = T(0.5) * ((uL[k] + uR[k]) + (d * (fL[k] - fR[k])));
-    S.flux(us, axis, xf, fs);
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        T lf = T(0.5) * ((fL[k] + fR[k]) + (c * (uL[k] - uR[k])));
-        F[k] = T(0.5) * (lf + fs[k]);
-    }
-}
-
-// ============================================================== GR source RK4 (FP64)
-// Fractional evolution on frozen neighbours, Solvers/BlackHoleEulerSolvers.cpp:159-232: slopes
-// from the neighbours at xc -/+ dx, face fluxes evaluated at xc -/+ dx (not dx/2), the middle
-// state advanced by frac * dt/dx and converted back at xc.
-CG_D void evolve_fraction_exact(const GRExact& S, double frac, const double* l, const double* m, const double* r,
-                                Pt xc, int axis, double dx, double dt, double w, int lim, double* out) {
-    double ul[5], um[5], ur[5], sl[5];
+CG_D void evolve_half_exact(const Sys& S, const T* l, const T* m, const T* r, Pt xc, int axis, double dx,
+                            const StepRatio& st, const Bias& w, int lim, T* left_face, T* right_face) {
+    T ul[5], um[5], ur[5];
     S.cons(l, shift_pt(xc, axis, -dx), ul);
     S.cons(m, xc, um);
     S.cons(r, shift_pt(xc, axis, dx), ur);
-    slope_exact(ul, um, ur, w, lim, sl);
-    double UL[5], UR[5], FL[5], FR[5];
+    evolve_half_cons(S, ul, um, ur, xc, axis, dx, st, w, lim, left_face, right_face);
+}
+
+// FORCE flux of two conserved states at interface xf (Solvers/EulerFirstOrderSolver.cpp:3-59;
+// GR Solvers/BlackHoleEulerFirstOrderSolver.cpp:3-47).
+template <class Sys, class T>
+CG_D void force_cons(const Sys& S, const T* uL, const T* uR, Pt xf, int axis, double dx, const StepRatio& st, T* F) {
+    T fL[5], fR[5], us[5], fs[5];
+    S.flux(uL, axis, shift_pt(xf, axis, -(dx * 0.5)), fL);
+    S.flux(uR, axis, shift_pt(xf, axis, dx * 0.5), fR);
+    const T c = T(st.c), d = T(st.d);
 #pragma unroll
-    for (int k = 0; k < 5; k++) { UL[k] = um[k] - (0.5 * sl[k]); UR[k] = um[k] + (0.5 * sl[k]); }
-    S.flux(UL, axis, shift_pt(xc, axis, -dx), FL);
-    S.flux(UR, axis, shift_pt(xc, axis, dx), FR);
-    const double s = frac * (dt / dx);
-    double nu[5];
+    for (int k = 0; k < 5; k++) {
+        us[k] = half((uL[k] + uR[k]) + (d * (fL[k] - fR[k])));
+        F[k] = half((fL[k] + fR[k]) + (c * (uL[k] - uR[k])));
+    }
+    S.flux(us, axis, xf, fs);
 #pragma unroll
-    for (int k = 0; k < 5; k++) nu[k] = um[k] + (s * (FL[k] - FR[k]));
-    S.prim(nu, xc, out);
+    for (int k = 0; k < 5; k++) F[k] = half(F[k] + fs[k]);
+}
+// ... of two primitive states
+template <class Sys, class T>
+CG_D void force_exact(const Sys& S, const T* L, const T* R, Pt xf, int axis, double dx, const StepRatio& st, T* F) {
+    T uL[5], uR[5];
+    S.cons(L, shift_pt(xf, axis, -(dx * 0.5)), uL);
+    S.cons(R, shift_pt(xf, axis, dx * 0.5), uR);
+    force_cons(S, uL, uR, xf, axis, dx, st, F);
+}
+
+// ============================================================== GR sweep and source step (FP64)
+// One interface flux of a black-hole sweep (Solvers/BlackHoleEulerSecondOrderSolver.cpp:3-37): the left
+// cell's right face from the evolution centred at xf - dx/2, the right cell's left face from that
+// centred at xf + dx/2, then FORCE at xf.  c: the four cells around the interface; order 1 takes the
+// two middle cells themselves.  The metric is formed once per point; the evolutions' centres are the
+// points where FORCE converts the face states.
+template <class T>
+CG_D void gr_interface(const GRExact* S, const V5<T>* c, int order, Pt xf, int axis, double dx, const StepRatio& st,
+                       const Bias& w, int lim, T* F) {
+    V5<T> uf[2], ff[2];  // conserved face states and their fluxes
+    Metric<T> gc;
+#pragma unroll 1
+    for (int side = 0; side < 2; side++) {
+        const Pt xc = shift_pt(xf, axis, side == 0 ? -(dx * 0.5) : dx * 0.5);
+        gr_metric(S, xc, &gc);
+        V5<T> face = c[1 + side];
+        if (order == 2) {
+            Metric<T> gm;
+            const V5<T> um = gr_cons(S, &gc, c[1 + side]);
+            gr_metric(S, shift_pt(xc, axis, -dx), &gm);
+            const V5<T> ul = gr_cons(S, &gm, c[side]);
+            gr_metric(S, shift_pt(xc, axis, dx), &gm);
+            const V5<T> ur = gr_cons(S, &gm, c[2 + side]);
+            V5<T> UL, UR;
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                const T hs = half(limited_slope(um.v[k] - ul.v[k], ur.v[k] - um.v[k], w, lim));
+                UL.v[k] = um.v[k] - hs;
+                UR.v[k] = um.v[k] + hs;
+            }
+            // the face wanted lies at xc + dx/2 (left cell) or xc - dx/2 (right cell): its point last
+            const T s = half(T(st.d));
+            gr_metric(S, shift_pt(xc, axis, side == 0 ? -(dx * 0.5) : dx * 0.5), &gm);
+            const V5<T> fo = gr_flux(S, &gm, side == 0 ? UL : UR, axis);
+            gr_metric(S, shift_pt(xc, axis, side == 0 ? dx * 0.5 : -(dx * 0.5)), &gm);
+            V5<T> U = side == 0 ? UR : UL;
+            const V5<T> fi = gr_flux(S, &gm, U, axis);
+#pragma unroll
+            for (int k = 0; k < 5; k++)
+                U.v[k] = U.v[k] + (s * (side == 0 ? fo.v[k] - fi.v[k] : fi.v[k] - fo.v[k]));
+            face = gr_prim(S, &gm, U);
+        }
+        uf[side] = gr_cons(S, &gc, face);
+        ff[side] = gr_flux(S, &gc, uf[side], axis);
+    }
+    V5<T> us;
+    const T cc = T(st.c), d = T(st.d);
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        us.v[k] = half((uf[0].v[k] + uf[1].v[k]) + (d * (ff[0].v[k] - ff[1].v[k])));
+        F[k] = half((ff[0].v[k] + ff[1].v[k]) + (cc * (uf[0].v[k] - uf[1].v[k])));
+    }
+    gr_metric(S, xf, &gc);
+    const V5<T> fs = gr_flux(S, &gc, us, axis);
+#pragma unroll
+    for (int k = 0; k < 5; k++) F[k] = half(F[k] + fs.v[k]);
+}
+
+// computeFORCEUpdate (Solvers/EulerFirstOrderSolver.cpp:96-101) of a black-hole cell at q.
+template <class T>
+CG_D void gr_update(const GRExact* S, const V5<T>& c, const T* FL, const T* FR, Pt q, double d, T* out) {
+    Metric<T> g;
+    gr_metric(S, q, &g);
+    V5<T> u = gr_cons(S, &g, c);
+#pragma unroll
+    for (int k = 0; k < 5; k++) u.v[k] = u.v[k] + (T(d) * (FL[k] - FR[k]));
+    give(gr_prim(S, &g, u), out);
+}
+
+// Fractional evolution on frozen neighbours, Solvers/BlackHoleEulerSolvers.cpp:159-232: slopes
+// from the neighbours at xc -/+ dx, face fluxes evaluated at xc -/+ dx (not dx/2), the middle
+// state advanced by frac * dt/dx and converted back at xc.  ul, ur: the neighbours' conserved
+// states, gl, gr_, gm the metrics there and at xc.
+template <class T>
+CG_D V5<T> evolve_fraction_in(const GRExact* S, double frac, const V5<T>& ul, const V5<T>& m, const V5<T>& ur,
+                              const Metric<T>* gl, const Metric<T>* gm, const Metric<T>* gr_, int axis,
+                              const StepRatio& st, const Bias& w, int lim) {
+    V5<T> um = gr_cons(S, gm, m), UL, UR;
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        const T hs = half(limited_slope(um.v[k] - ul.v[k], ur.v[k] - um.v[k], w, lim));
+        UL.v[k] = um.v[k] - hs;
+        UR.v[k] = um.v[k] + hs;
+    }
+    UL = gr_flux(S, gl, UL, axis);
+    UR = gr_flux(S, gr_, UR, axis);
+    const T s = T(frac) * T(st.d);
+#pragma unroll
+    for (int k = 0; k < 5; k++) um.v[k] = um.v[k] + (s * (UL.v[k] - UR.v[k]));
+    return gr_prim(S, gm, um);
+}
+template <class T>
+CG_D void evolve_fraction_exact(const GRExact& S, double frac, const T* l, const T* m, const T* r, Pt xc, int axis,
+                                double dx, const StepRatio& st, const Bias& w, int lim, T* out) {
+    Metric<T> gl, gm, gr_;
+    gr_metric(&S, shift_pt(xc, axis, -dx), &gl);
+    gr_metric(&S, xc, &gm);
+    gr_metric(&S, shift_pt(xc, axis, dx), &gr_);
+    give(evolve_fraction_in(&S, frac, gr_cons(&S, &gl, five(l)), five(m), gr_cons(&S, &gr_, five(r)), &gl, &gm, &gr_,
+                            axis, st, w, lim), out);
 }
 
 // Classical RK4 on the source with interleaved fractional sweeps,
 // Solvers/BlackHoleEulerForcingSolver.cpp:3-70 (1D: X fractions 1/2, 1/2, 1) and :72-185
 // (2D: X 1/4, Y 1/2, X 1/4 for stages 1-2; X 1/2, Y 1, X 1/2 for stage 3).
-// cl..cb are the conserved neighbours (cell-centred), q the cell's coordinate; returns the
-// updated conserved state.
-CG_D void rk_cell_exact(const GRExact& S, int dims, const double* cl, const double* cm, const double* cr,
-                        const double* ct, const double* cb, Pt q, double dx, double dt, double w, int lim,
-                        double* out) {
-    double L[5], R[5], Tp[5], B[5];
-    S.prim(cl, shift_pt(q, 0, -dx), L);
-    S.prim(cr, shift_pt(q, 0, dx), R);
-    if (dims == 2) {
-        S.prim(ct, shift_pt(q, 1, -dx), Tp);
-        S.prim(cb, shift_pt(q, 1, dx), B);
+// u: conserved states of the left, right, top and bottom neighbours and (u[4]) of the cell itself
+// (cell-centred); q the cell's coordinate; returns the updated conserved state.  The neighbours are
+// frozen and the spacetime is static: the neighbours' states as the fractional sweeps read them
+// (conserved again from their recovered primitives), the metrics and the source term's metric part
+// are formed once for the four stages.
+template <class T>
+CG_D V5<T> rk_cell_exact(const GRExact* S, int dims, const V5<T>* u, Pt q, double dx, double dt, const StepRatio& sr,
+                         const Bias& w, int lim, Metric<T>* gq) {
+    Metric<T> gn[4];
+    SourceMetric<T> sm;
+    V5<T> un[4];
+#pragma unroll 1
+    for (int n = 0; n < (dims == 2 ? 4 : 2); n++) {
+        gr_metric(S, shift_pt(q, n >> 1, n & 1 ? dx : -dx), &gn[n]);
+        un[n] = gr_cons(S, &gn[n], gr_prim(S, &gn[n], u[n]));
     }
-    double k[4][5];
-    {
-        double s[5];
-        S.source(cm, q, s);
+    gr_metric(S, q, gq);
+    gr_source_metric(S, q, gq->al, &sm);
+    const V5<T> cm = u[4];
+    // out = cm + (k0 + (2 k1 + (2 k2 + k3))) / 6; the stages share one copy of the code
+    V5<T> k0, k1, k2, k = gr_source(S, gq, &sm, cm);
 #pragma unroll
-        for (int i = 0; i < 5; i++) k[0][i] = dt * s[i];
-    }
+    for (int i = 0; i < 5; i++) k0.v[i] = k1.v[i] = k2.v[i] = k.v[i] = T(dt) * k.v[i];
+#pragma unroll 1
     for (int stage = 0; stage < 3; stage++) {
-        double st[5], Mp[5], E[5], c[5], s[5];
+        V5<T> p;
 #pragma unroll
-        for (int i = 0; i < 5; i++) st[i] = stage < 2 ? (cm[i] + (0.5 * k[stage][i])) : (cm[i] + k[stage][i]);
-        S.prim(st, q, Mp);
-        if (dims == 1) {
-            const double fx = stage < 2 ? 0.5 : 1.0;
-            evolve_fraction_exact(S, fx, L, Mp, R, q, 0, dx, dt, w, lim, E);
-        } else {
-            const double fx = stage < 2 ? 0.25 : 0.5, fy = stage < 2 ? 0.5 : 1.0;
-            double E1[5], E2[5];
-            evolve_fraction_exact(S, fx, L, Mp, R, q, 0, dx, dt, w, lim, E1);
-            evolve_fraction_exact(S, fy, Tp, E1, B, q, 1, dx, dt, w, lim, E2);
-            evolve_fraction_exact(S, fx, L, E2, R, q, 0, dx, dt, w, lim, E);
+        for (int i = 0; i < 5; i++) p.v[i] = cm.v[i] + (stage < 2 ? half(k.v[i]) : k.v[i]);
+        p = gr_prim(S, gq, p);
+        const double fx = dims == 1 ? (stage < 2 ? 0.5 : 1.0) : (stage < 2 ? 0.25 : 0.5), fy = stage < 2 ? 0.5 : 1.0;
+#pragma unroll 1
+        for (int part = 0; part < (dims == 1 ? 1 : 3); part++) {
+            const int y = part == 1;
+            p = evolve_fraction_in(S, y ? fy : fx, un[2 * y], p, un[2 * y + 1], &gn[2 * y], gq, &gn[2 * y + 1], y, sr, w,
+                                   lim);
         }
-        S.cons(E, q, c);
-        S.source(c, q, s);
+        k = gr_source(S, gq, &sm, gr_cons(S, gq, p));
 #pragma unroll
-        for (int i = 0; i < 5; i++) k[stage + 1][i] = dt * s[i];
+        for (int i = 0; i < 5; i++) {
+            k.v[i] = T(dt) * k.v[i];
+            if (stage == 0) k1.v[i] = twice(k.v[i]);
+            else if (stage == 1) k2.v[i] = twice(k.v[i]);
+        }
     }
+    V5<T> o;
 #pragma unroll
-    for (int i = 0; i < 5; i++) out[i] = cm[i] + ((1.0 / 6.0) * (k[0][i] + ((2.0 * k[1][i]) + ((2.0 * k[2][i]) + k[3][i]))));
+    for (int i = 0; i < 5; i++) o.v[i] = cm.v[i] + (T(1.0 / 6.0) * (k0.v[i] + (k1.v[i] + (k2.v[i] + k.v[i]))));
+    return o;
 }
 
 }  // namespace cg

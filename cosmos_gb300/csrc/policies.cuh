@@ -25,110 +25,155 @@ struct LineMap {
 };
 
 // ------------------------------------------------------------------ reference-exact, FP64
-// Primitive storage exactly like the reference's grids.  Sys = NewtonExact<double>, SRExact or
-// GRExact.  Coordinate-free systems share one half-step evolution per cell (both faces);
-// GR evolves each face at its own, separately rounded, coordinate.
+// The stages of a sweep in hardware FP64, out of line: taken where a stage's integer-pipe results are
+// not all finite (exact_math.cuh).  Arguments go by value, so that the callers' stay in registers.
+template <class Sys>
+__device__ __noinline__ V5<double> slow_cons(Sys S, V5<double> p) {
+    V5<double> u;
+    S.cons(p.v, Pt{0.0, 0.0, 0.0}, u.v);
+    return u;
+}
+struct FacePair { V5<double> L, R; };
+template <class Sys>
+__device__ __noinline__ FacePair slow_faces(Sys S, V5<double> l, V5<double> m, V5<double> r, int axis, StepRatio st,
+                                            Bias w, int lim) {
+    const Pt z{0.0, 0.0, 0.0};
+    double a[5], b[5];
+    FacePair o;
+    evolve_half_cons(S, l.v, m.v, r.v, z, axis, 0.0, st, w, lim, a, b);
+    S.cons(a, z, o.L.v);
+    S.cons(b, z, o.R.v);
+    return o;
+}
+template <class Sys>
+__device__ __noinline__ V5<double> slow_force(Sys S, V5<double> uL, V5<double> uR, int axis, StepRatio st) {
+    V5<double> o;
+    force_cons(S, uL.v, uR.v, Pt{0.0, 0.0, 0.0}, axis, 0.0, st, o.v);
+    return o;
+}
+template <class Sys>
+__device__ __noinline__ V5<double> slow_update(Sys S, V5<double> u, V5<double> FL, V5<double> FR, double d) {
+    V5<double> o;
+    for (int f = 0; f < 5; f++) u.v[f] = u.v[f] + (d * (FL.v[f] - FR.v[f]));
+    S.prim(u.v, Pt{0.0, 0.0, 0.0}, o.v);
+    return o;
+}
+template <class Sys>
+__device__ __noinline__ double slow_wavespeed(Sys S, V5<double> c, int dims, Pt q) {
+    if constexpr (Sys::kCoords) return S.sound_speed(c.v, q);
+    else return S.wavespeed(c.v, dims, q);
+}
+
+CG_D void load5(const double* a, xd* o) {
+#pragma unroll
+    for (int f = 0; f < 5; f++) o[f] = xd(a[f]);
+}
+CG_D void store5(const xd* a, double* o) {
+#pragma unroll
+    for (int f = 0; f < 5; f++) o[f] = a[f].v;
+}
+
+// The stages of a coordinate-free sweep on conserved states (Newtonian, SR).
+template <class Sys>
+struct ExactStages {
+    Sys sys;
+    Bias w;
+    int lim;
+    // conserved state of a cell
+    CG_D V5<double> cons(const V5<double>& p) const {
+        xd a[5], u[5];
+        V5<double> o;
+        load5(p.v, a);
+        sys.cons(a, Pt{0.0, 0.0, 0.0}, u);
+        store5(u, o.v);
+        if (any_nonfinite(u, 5)) o = slow_cons(sys, p);
+        return o;
+    }
+    // conserved face states of the cell m after its half-step evolution (each through its primitives, as
+    // the reference's evolved states are)
+    CG_D void faces(const V5<double>& l, const V5<double>& m, const V5<double>& r, int axis, const StepRatio& st,
+                    V5<double>& L, V5<double>& R) const {
+        const Pt z{0.0, 0.0, 0.0};
+        xd a[5], b[5], c[5], fl[5], fr[5];
+        load5(l.v, a);
+        load5(m.v, b);
+        load5(r.v, c);
+        evolve_half_cons(sys, a, b, c, z, axis, 0.0, st, w, lim, fl, fr);
+        sys.cons(fl, z, a);
+        sys.cons(fr, z, b);
+        store5(a, L.v);
+        store5(b, R.v);
+        if (any_nonfinite(a, 5) || any_nonfinite(b, 5)) {
+            const FacePair o = slow_faces(sys, l, m, r, axis, st, w, lim);
+            L = o.L;
+            R = o.R;
+        }
+    }
+    CG_D V5<double> force(const V5<double>& uL, const V5<double>& uR, int axis, const StepRatio& st) const {
+        xd a[5], b[5], f[5];
+        V5<double> o;
+        load5(uL.v, a);
+        load5(uR.v, b);
+        force_cons(sys, a, b, Pt{0.0, 0.0, 0.0}, axis, 0.0, st, f);
+        store5(f, o.v);
+        if (any_nonfinite(f, 5)) o = slow_force(sys, uL, uR, axis, st);
+        return o;
+    }
+    // computeFORCEUpdate, Solvers/EulerFirstOrderSolver.cpp:96-101, then setConservedVariableVector
+    CG_D V5<double> update(const V5<double>& u, const V5<double>& FL, const V5<double>& FR, double d) const {
+        xd a[5], p[5];
+        V5<double> o;
+#pragma unroll
+        for (int f = 0; f < 5; f++) a[f] = xd(u.v[f]) + (xd(d) * xd(FL.v[f] - FR.v[f]));
+        sys.prim(a, Pt{0.0, 0.0, 0.0}, p);
+        store5(p, o.v);
+        if (any_nonfinite(p, 5)) o = slow_update(sys, u, FL, FR, d);
+        return o;
+    }
+    CG_D double wavespeed(const V5<double>& c, int dims) const {
+        xd p[5];
+        load5(c.v, p);
+        double s = sys.wavespeed(p, dims, Pt{0.0, 0.0, 0.0}).v;
+        if (!xm::finite(s)) s = slow_wavespeed(sys, c, dims, Pt{0.0, 0.0, 0.0});
+        return speed_or_inf(c.v[0], c.v[4], s);
+    }
+};
+
+// Primitive storage exactly like the reference's grids, for the generic kernels: the FP64 batch's tiles
+// (Newtonian) and the CFL reduction of every system.  The single grids' sweeps are in exact_tiles.cuh.
 template <class Sys>
 struct ExactPolicy {
     using S = double;
     using X = double;
     using W = double;  // wavespeed reduction type
     using Cell = V5<double>;
-    using Face = V5<double>;
-    struct Coef { double dt; };
-    static constexpr bool kShared = !Sys::kCoords;
-    static constexpr bool kMasked = true;
+    using Face = V5<double>;  // conserved
+    struct Coef { double dt; StepRatio r; };
+    static constexpr bool kMasked = false;
     static constexpr bool kHasDx = true;
-    Sys sys;
+    ExactStages<Sys> st;
     LineMap lm;
-    int dims, order, ny;
-    double dx, dt, w;
-    int lim;
-    int capped;
+    int dims, ny;
+    double dx, dt;
+    StepRatio r;
 
-    CG_D Coef make_coef(const DtSrc&, double d) const { return Coef{d}; }
-    CG_D void use_coef(const Coef& c) { dt = c.dt; capped = 0; sys.capped = &capped; }
-    CG_D Pt cell_pt(int line, int k) const {
-        int i, j;
-        lm.ij(line, k, i, j);
-        return Pt{j * dx, i * dx, 0.0};
+    CG_D Coef make_coef(const DtSrc& ds, double d) const { return Coef{d, ds.ratio(d, dx)}; }
+    CG_D void use_coef(const Coef& c) { dt = c.dt; r = c.r; }
+    CG_D void recon(const Cell& l, const Cell& m, const Cell& rr, int, int, Face& L, Face& R) const {
+        st.faces(st.cons(l), st.cons(m), st.cons(rr), lm.axis, r, L, R);
     }
-    // interface between cells f-1 and f: (f - 0.5) dx along the sweep axis
-    CG_D Pt face_pt(int line, int f) const {
-        if (lm.axis == 0) return Pt{(f - 0.5) * dx, line * dx, 0.0};
-        return Pt{line * dx, (f - 0.5) * dx, 0.0};
+    CG_D void face_of(const Cell& c, Face& f) const { f = st.cons(c); }
+    CG_D void flux(const Face& L, const Face& R, int, int, V5<double>& F) const { F = st.force(L, R, lm.axis, r); }
+    CG_D Cell update(const Cell& c, const V5<double>& FL, const V5<double>& FR, int, int) const {
+        return st.update(st.cons(c), FL, FR, r.d);
     }
-    CG_D void recon(const Cell& l, const Cell& m, const Cell& r, int, int, Face& L, Face& R) const {
-        evolve_half_exact(sys, l.v, m.v, r.v, Pt{0.0, 0.0, 0.0}, lm.axis, dx, dt, w, lim, L.v, R.v);
-    }
-    // GR: the left cell of interface f evolves at xf - dx/2, the right cell at xf + dx/2
-    // (Solvers/BlackHoleEulerSecondOrderSolver.cpp:3-37)
-    CG_D void recon_side(const Cell& l, const Cell& m, const Cell& r, int line, int k, int side, Face& o) const {
-        if (side == 1) {
-            Pt xc = shift_pt(face_pt(line, k + 1), lm.axis, -(dx * 0.5));
-            evolve_half_exact(sys, l.v, m.v, r.v, xc, lm.axis, dx, dt, w, lim, (double*)nullptr, o.v);
-        } else {
-            Pt xc = shift_pt(face_pt(line, k), lm.axis, dx * 0.5);
-            evolve_half_exact(sys, l.v, m.v, r.v, xc, lm.axis, dx, dt, w, lim, o.v, (double*)nullptr);
-        }
-    }
-    CG_D void face_of(const Cell& c, Face& f) const { f = c; }
-    CG_D void flux(const Face& L, const Face& R, int line, int f, V5<double>& F) const {
-        force_exact(sys, L.v, R.v, face_pt(line, f), lm.axis, dx, dt, F.v);
-    }
-    // computeFORCEUpdate, Solvers/EulerFirstOrderSolver.cpp:96-101, then setConservedVariableVector
-    CG_D Cell update(const Cell& c, const V5<double>& FL, const V5<double>& FR, int line, int k) const {
-        Pt q = cell_pt(line, k);
-        double u[5], nu[5];
-        sys.cons(c.v, q, u);
-        const double d = dt / dx;
-#pragma unroll
-        for (int f = 0; f < 5; f++) nu[f] = u[f] + (d * (FL.v[f] - FR.v[f]));
-        Cell o;
-        sys.prim(nu, q, o.v);
-        return o;
-    }
-    CG_D bool excised_stencil(int line, int k) const;
-    CG_D bool active(int line, int k, const unsigned char* mask) const {
-        if (!lm.mask_on(mask, line, k)) return false;
-        if (Sys::kCoords) return !excised_stencil(line, k);
-        return true;
-    }
+    CG_D bool active(int, int, const unsigned char*) const { return true; }
     CG_D double wavespeed(const Cell& c, int line, int k) const;
-    CG_D void flush_status(int* st) const {
-        if (st && capped) atomicOr(st, ST_NEWTON_CAP);
-    }
+    CG_D void flush_status(int*) const {}
 };
 
 template <class Sys>
-CG_D bool ExactPolicy<Sys>::excised_stencil(int, int) const { return false; }
-template <class Sys>
-CG_D double ExactPolicy<Sys>::wavespeed(const Cell& c, int, int) const {
-    return speed_or_inf(c.v[0], c.v[4], sys.wavespeed(c.v, dims, Pt{0, 0, 0}));
-}
-
-// GR excision: the updated cell and its stencil along both axes must lie outside the horizon
-// (Solvers/BlackHoleEulerSecondOrderSolver.cpp:44-46 in 1D, :81-85 in 2D; reach 1 for FORCE,
-// Solvers/BlackHoleEulerFirstOrderSolver.cpp:94-95, :131-133).
-template <>
-CG_D bool ExactPolicy<GRExact>::excised_stencil(int line, int k) const {
-    int i, j;
-    lm.ij(line, k, i, j);
-    const int reach = order == 2 ? 2 : 1;
-    const BHExact& b = sys.bh;
-    if (dims == 1) {
-        for (int d = -reach; d <= reach; d++)
-            if (b.excised((j + d) * dx, 0.0, 0.0)) return true;
-        return false;
-    }
-    if (b.excised(j * dx, i * dx, 0.0)) return true;
-    for (int d = 1; d <= reach; d++) {
-        if (b.excised((j - d) * dx, i * dx, 0.0) || b.excised((j + d) * dx, i * dx, 0.0) ||
-            b.excised(j * dx, (i - d) * dx, 0.0) || b.excised(j * dx, (i + d) * dx, 0.0))
-            return true;
-    }
-    return false;
-}
+CG_D double ExactPolicy<Sys>::wavespeed(const Cell& c, int, int) const { return st.wavespeed(c, dims); }
 
 // GR CFL speed, Solvers/BlackHoleEulerSolvers.cpp:87-131: coordinates use spacing 1/N, and in 2D
 // the excision test reads (j/ncol, i/nrow) while the speed is evaluated at (i/nrow, j/ncol).
@@ -136,14 +181,16 @@ template <>
 CG_D double ExactPolicy<GRExact>::wavespeed(const Cell& c, int line, int k) const {
     int i, j;
     lm.ij(line, k, i, j);
-    if (dims == 1) {
-        const double cs = 1.0 / lm.nx;
-        if (sys.bh.excised(j * cs, 0.0, 0.0)) return 0.0;
-        return speed_or_inf(c.v[0], c.v[4], fabs(sys.sound_speed(c.v, Pt{j * cs, 0.0, 0.0})));
-    }
-    const double rs = 1.0 / ny, cs = 1.0 / lm.nx;
-    if (sys.bh.excised(j * cs, i * rs, 0.0)) return 0.0;
-    return speed_or_inf(c.v[0], c.v[4], fabs(sys.sound_speed(c.v, Pt{i * rs, j * cs, 0.0})));
+    const double cs = quotient(1.0, (double)lm.nx), rs = dims == 1 ? 0.0 : quotient(1.0, (double)ny);
+    const double x = j * cs, y = i * rs;
+    const GRExact& sys = st.sys;
+    if (sys.bh.excised(x, y, 0.0)) return 0.0;
+    const Pt q = dims == 1 ? Pt{x, 0.0, 0.0} : Pt{y, x, 0.0};
+    xd p[5];
+    load5(c.v, p);
+    double s = sys.sound_speed(p, q).v;
+    if (!xm::finite(s)) s = slow_wavespeed(sys, c, dims, q);
+    return speed_or_inf(c.v[0], c.v[4], fabs(s));
 }
 
 // ------------------------------------------------------------------ Newtonian FP32 bulk
@@ -157,7 +204,6 @@ struct NewtonFastPolicy {
     using Cell = V5<float>;
     using Face = V5<float>;
     using Coef = FastCoef;
-    static constexpr bool kShared = true;
     static constexpr bool kMasked = MASKED;
     static constexpr bool kHasDx = false;  // dx enters through the precomputed coefficients
     NewtonFastParams P;
@@ -176,7 +222,6 @@ struct NewtonFastPolicy {
     CG_D void recon(const Cell& l, const Cell& m, const Cell& r, int, int, Face& L, Face& R) const {
         nf_recon<AXIS, LIM>(P, l.v, m.v, r.v, half_dtdx, L.v, R.v);
     }
-    CG_D void recon_side(const Cell&, const Cell&, const Cell&, int, int, int, Face&) const {}
     CG_D void face_of(const Cell& c, Face& f) const { f = c; }
     CG_D void flux(const Face& L, const Face& R, int, int, V5<float>& F) const {
         nf_force<AXIS>(P, L.v, R.v, half_dtdx, q_dxdt, F.v);
@@ -203,7 +248,6 @@ struct SRFastPolicy {
     using Cell = V5<float>;
     using Face = V5<float>;
     using Coef = FastCoef;
-    static constexpr bool kShared = true;
     static constexpr bool kMasked = MASKED;
     static constexpr bool kHasDx = false;
     NewtonFastParams NP;  // limiter and bias factors
@@ -222,7 +266,6 @@ struct SRFastPolicy {
     CG_D void recon(const Cell& l, const Cell& m, const Cell& r, int, int, Face& L, Face& R) {
         sr_recon_fast<AXIS, LIM>(P, NP, l.v, m.v, r.v, half_dtdx, L.v, R.v, &flags);
     }
-    CG_D void recon_side(const Cell&, const Cell&, const Cell&, int, int, int, Face&) const {}
     CG_D void face_of(const Cell& c, Face& f) const { f = c; }
     CG_D void flux(const Face& L, const Face& R, int, int, V5<float>& F) {
         sr_force_fast<AXIS>(P, L.v, R.v, half_dtdx, q_dxdt, F.v, &flags);

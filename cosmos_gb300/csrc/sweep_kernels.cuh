@@ -25,14 +25,25 @@ struct DtSrc {
     double scale;
     int nsub;        // > 0 selects 0.5 * (dt / nsub)
     int fsel;        // FP32 coefficients: controller slot (0: dt, 1: dt/2)
-    FastCoef ffix;   // FP32 coefficients of `fixed`, formed on the host
+    FastCoef ffix;   // coefficients of `fixed`, formed on the host (FP32, FP64)
+    StepRatio xfix;
     CG_D bool get(double& dt) const {
         if (!ctl) { dt = fixed; return true; }
         if (!ctl->active) return false;
-        dt = nsub > 0 ? 0.5 * (ctl->dt / nsub) : ctl->dt * scale;
+        dt = nsub > 0 ? 0.5 * (nsub > 1 ? ctl->dt / nsub : ctl->dt) : ctl->dt * scale;
         return true;
     }
     CG_D FastCoef fast_coef() const { return ctl ? ctl->fc[fsel] : ffix; }
+    CG_D StepRatio ratio(double dt, double dx) const {
+        if (!ctl) return xfix;
+        if (nsub > 0) return StepRatio{quotient(dt, dx), quotient(dx, dt)};
+        return ctl->xr[fsel];
+    }
+    void set_fixed(double dt, double dx) {
+        fixed = dt;
+        ffix = make_fast_coef(dt, dx);
+        xfix = make_ratio(dt, dx);
+    }
 };
 
 // Output side of a sweep: fused wavespeed maximum (for the next step's dt) and status bits.
@@ -56,122 +67,6 @@ CG_D void store_cell(const typename Pol::Cell& c, typename Pol::S* dst, const Ge
     const size_t idx = (size_t)i * G.pitch + j;
 #pragma unroll
     for (int f = 0; f < 5; f++) dst[f * G.fstride + idx] = (typename Pol::S)c.v[f];
-}
-
-// ------------------------------------------------------------------ X sweep: one row tile
-// NT threads; cells s0-2 .. s0+NT-1 staged in shared memory; NT half-step evolutions,
-// NT-1 interface fluxes, NT-2 updates per block.
-template <class Pol, int ORDER, int NT>
-__global__ void __launch_bounds__(NT) sweep_x_kernel(Pol pol, Geom G, const typename Pol::S* __restrict__ src,
-                                                     typename Pol::S* __restrict__ dst, DtSrc ds, SweepOut out) {
-    using X = typename Pol::X;
-    constexpr int TS = NT - 2;
-    __shared__ X sc[5][NT + 2];
-    __shared__ X sl[5][NT];
-    __shared__ X sr[5][NT];
-    __shared__ X sf[5][NT];
-    const int t = threadIdx.x;
-    const int row = blockIdx.y;
-    const int s0 = blockIdx.x * TS;
-    const int n = G.nx;
-    const int send = min(s0 + TS, n);  // one past the last updated cell
-    // the step's coefficients are formed once per block (FP64 work is 1/64 rate on GB300)
-    __shared__ typename Pol::Coef s_coef;
-    __shared__ int s_act;
-    if (t == 0) {
-        double dt;
-        s_act = ds.get(dt);
-        if (s_act) s_coef = pol.make_coef(ds, dt);
-    }
-    __syncthreads();
-    const bool act = s_act != 0;
-    if (!act) {  // inactive step: keep the ping-pong buffers consistent
-        if (s0 + t < send) {
-            typename Pol::Cell c;
-            load_cell(pol, src, G, row, s0 + t, c);
-            store_cell<Pol>(c, dst, G, row, s0 + t);
-        }
-        return;
-    }
-    pol.use_coef(s_coef);
-    // stage cells s0-2+t (and two more) with ghost mapping along x
-    for (int q = t; q < NT + 2; q += NT) {
-        const int k = s0 - 2 + q;
-        if (k <= send + 1) {
-            typename Pol::Cell c;
-            load_cell(pol, src, G, row, ghost_index(k, n, G.bc), c);
-#pragma unroll
-            for (int f = 0; f < 5; f++) sc[f][q] = c.v[f];
-        }
-    }
-    __syncthreads();
-    auto cell_at = [&](int q, typename Pol::Cell& c) {
-#pragma unroll
-        for (int f = 0; f < 5; f++) c.v[f] = sc[f][q];
-    };
-    // interface s0+t lies between cells s0+t-1 and s0+t; needed when either side updates
-    auto iface_needed = [&](int fi) {
-        if (fi < s0 || fi > send) return false;
-        const bool a = fi - 1 >= s0 && pol.active(row, fi - 1, out.mask);
-        const bool b = fi < send && pol.active(row, fi, out.mask);
-        return a || b;
-    };
-    if (ORDER == 2 && Pol::kShared) {
-        // half-step evolution of cell s0-1+t from smem cells t, t+1, t+2
-        const int k = s0 - 1 + t;
-        if (k <= send && (iface_needed(k) || iface_needed(k + 1))) {
-            typename Pol::Cell a, b, c;
-            typename Pol::Face L, R;
-            cell_at(t, a); cell_at(t + 1, b); cell_at(t + 2, c);
-            pol.recon(a, b, c, row, k, L, R);
-#pragma unroll
-            for (int f = 0; f < 5; f++) { sl[f][t] = L.v[f]; sr[f][t] = R.v[f]; }
-        }
-        __syncthreads();
-    }
-    {
-        const int fi = s0 + t;
-        if (t < NT - 1 && iface_needed(fi)) {
-            typename Pol::Face L, R;
-            if (ORDER == 1) {
-                typename Pol::Cell a, b;
-                cell_at(t + 1, a); cell_at(t + 2, b);
-                pol.face_of(a, L); pol.face_of(b, R);
-            } else if (Pol::kShared) {
-#pragma unroll
-                for (int f = 0; f < 5; f++) { L.v[f] = sr[f][t]; R.v[f] = sl[f][t + 1]; }
-            } else {
-                typename Pol::Cell a, b, c, d;
-                cell_at(t, a); cell_at(t + 1, b); cell_at(t + 2, c); cell_at(t + 3, d);
-                pol.recon_side(a, b, c, row, fi - 1, 1, L);
-                pol.recon_side(b, c, d, row, fi, 0, R);
-            }
-            V5<X> F;
-            pol.flux(L, R, row, fi, F);
-#pragma unroll
-            for (int f = 0; f < 5; f++) sf[f][t] = F.v[f];
-        }
-    }
-    __syncthreads();
-    typename Pol::W w = 0;
-    unsigned long long* const wslot = out.slot();
-    const int k = s0 + t;
-    if (t < TS && k < send) {
-        typename Pol::Cell c, nc;
-        cell_at(t + 2, c);
-        if (pol.active(row, k, out.mask)) {
-            V5<X> FL, FR;
-#pragma unroll
-            for (int f = 0; f < 5; f++) { FL.v[f] = sf[f][t]; FR.v[f] = sf[f][t + 1]; }
-            nc = pol.update(c, FL, FR, row, k);
-        } else {
-            nc = c;
-        }
-        store_cell<Pol>(nc, dst, G, row, k);
-        if (wslot) w = pol.wavespeed(nc, row, k);
-    }
-    if (wslot) block_max_to<NT>(wslot, w);
-    pol.flush_status(out.status);
 }
 
 // ------------------------------------------------------------------ X sweep, cell ownership
@@ -352,11 +247,11 @@ CG_D typename Pol::W y_march_seg(Pol& pol, const Geom& G, const typename Pol::S*
         Cell cm2, cm1, c0, c1, c2;
         ld(y0 - 2, cm2); ld(y0 - 1, cm1); ld(y0, c0); ld(y0 + 1, c1);
         V5<X> Fp, Fn;
-        Face R0;  // right face of the current cell (shared recon)
+        Face R0;  // right face of the current cell
         bool nf_next = msk ? need(y0 + 1) : true;
         if (ORDER == 1) {
             if (need(y0)) { Face L, R; pol.face_of(cm1, L); pol.face_of(c0, R); pol.flux(L, R, j, y0, Fp); }
-        } else if (Pol::kShared) {
+        } else {
             Face Lm1, Rm1, L0;
             if (need(y0)) {
                 pol.recon(cm2, cm1, c0, j, y0 - 1, Lm1, Rm1);
@@ -365,13 +260,6 @@ CG_D typename Pol::W y_march_seg(Pol& pol, const Geom& G, const typename Pol::S*
             } else if (nf_next) {
                 pol.recon(cm1, c0, c1, j, y0, L0, R0);
             }
-        } else {
-            if (need(y0)) {
-                Face L, R;
-                pol.recon_side(cm2, cm1, c0, j, y0 - 1, 1, L);
-                pol.recon_side(cm1, c0, c1, j, y0, 0, R);
-                pol.flux(L, R, j, y0, Fp);
-            }
         }
         for (int y = y0; y < y1; y++) {
             ld(y + 2, c2);
@@ -379,25 +267,18 @@ CG_D typename Pol::W y_march_seg(Pol& pol, const Geom& G, const typename Pol::S*
             if (msk) nf_next = need(y + 2);
             if (ORDER == 1) {
                 if (nf) { Face L, R; pol.face_of(c0, L); pol.face_of(c1, R); pol.flux(L, R, j, y + 1, Fn); }
-            } else if (Pol::kShared) {
+            } else {
                 Face L1, R1;
                 if (nf || nf_next) pol.recon(c0, c1, c2, j, y + 1, L1, R1);  // R1 is read only if nf_next
                 if (nf) pol.flux(R0, L1, j, y + 1, Fn);
                 R0 = R1;
-            } else {
-                if (nf) {
-                    Face L, R;
-                    pol.recon_side(cm1, c0, c1, j, y, 1, L);
-                    pol.recon_side(c0, c1, c2, j, y + 1, 0, R);
-                    pol.flux(L, R, j, y + 1, Fn);
-                }
             }
             Cell nc = c0;
             if (pol.active(j, y, out.mask)) nc = pol.update(c0, Fp, Fn, j, y);
             store_cell<Pol>(nc, dst, G, y, j);
             if (want_w) { const typename Pol::W ws = pol.wavespeed(nc, j, y); w = (ws > w) ? ws : w; }
             Fp = Fn;
-            cm1 = c0; c0 = c1; c1 = c2;
+            c0 = c1; c1 = c2;
         }
     }
     pol.flush_status(out.status);
