@@ -8,8 +8,8 @@
 // 400 warps on 152 SMs.  Each cell's conserved state is formed once and read by its neighbours from
 // shared memory (before: three times in registers), each half-step evolution and each interface flux once
 // per tile.  Measured with the integer-pipe arithmetic (GB300, whole solves against the marching,
-// hardware-FP64 form): 389 x 509 Newtonian SLIC 0.50 -> 0.15 ms per sweep, 200 x 200 FORCE 0.113 -> 0.021,
-// 181 x 230 SR 0.88 -> 0.14, 150 x 150 black-hole step 9.0 -> 3.1 ms, 128^2 Level-1 AMR run 79.5 -> 16.3 ms.
+// hardware-FP64 form): 389 x 509 Newtonian SLIC 0.50 -> 0.10 ms per sweep, 200 x 200 FORCE 0.113 -> 0.017,
+// 181 x 230 SR 0.88 -> 0.11, 150 x 150 black-hole step 9.0 -> 2.6 ms, 128^2 Level-1 AMR run 79.5 -> 13.8 ms.
 #pragma once
 #include "policies.cuh"
 
@@ -63,8 +63,10 @@ template <int N> CG_D void sm_set(double (&a)[5][N], int t, const V5<double>& c)
 // ---- coordinate-free systems (Newtonian, SR).  Position p owns cell c = s0 - 1 + p: its conserved state,
 // its half-step evolution and the flux at its right interface; positions 1 .. P - 2 update.  MASKED (AMR
 // levels): cells whose flag is off are copied, and only what an updating cell needs is evaluated.
+// Four blocks of 128 threads per SM (at most 128 registers): 3, 5 or 6 measured within 3 %, so occupancy is
+// not what bounds them.
 template <class Sys, int AXIS, int ORDER, int NT, int LC, bool MASKED>
-__global__ void __launch_bounds__(NT) exact_tile_kernel(const __grid_constant__ ExactStages<Sys> S, TileArgs A) {
+__global__ void __launch_bounds__(NT, 512 / NT) exact_tile_kernel(const __grid_constant__ ExactStages<Sys> S, TileArgs A) {
     constexpr int P = NT / LC;
     __shared__ double sU[5][NT + 2 * LC];  // conserved states of cells s0 - 2 .. s0 + P - 1
     __shared__ double sL[5][NT];           // conserved left-face state of the thread's cell

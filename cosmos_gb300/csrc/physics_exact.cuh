@@ -51,27 +51,36 @@ CG_D double limited_slope(double dl, double dr, const Bias& w, int lim) {
 // the smaller numerator (van Leer 2 min(r, 1) / (1 + r); SuperBee and MinBee 2 / (1 + r) from r = 1
 // on).  Both differences inside the clamp (uniform flow, a velocity that is zero everywhere) give
 // r = 1 and a limiter of 1.
+// Bounds: differences zero or in [2^-200, 2^101) (tested); r in [2^-118, 2^118] after the clamp; the
+// candidates in [2^-120, 2^120]; the slope zero or at least 2^-320.
 CG_D xd limited_slope(xd dl, xd dr, const Bias& w, int lim) {
-    const bool plain = w.w == 0.0;
-    const xd s = plain ? half(dl) + half(dr) : (xd(w.a) * dl) + (xd(w.b) * dr);
-    const bool tl = nearer_zero(dl, 1e-5), tr = nearer_zero(dr, 1e-5);
-    if (tl && tr && plain) return s;
-    const xd r = (tl ? xd(1e-5) : dl) / (tr ? xd(1e-5) : dr);
-    if (xm::plain_negative(r.v)) return xm::finite(s.v) ? xd(xm::double_of(xm::bits_of(s.v) & 0x8000000000000000ull)) : s;
-    if (!xm::plain_positive(r.v)) return xd(xm::double_of(0x7ff8000000000000ull));
-    const bool lt1 = below(r, 1.0);
-    if (plain) {
-        xd phi = xd(2.0);
+    const xr l = xr(dl.v), r_ = xr(dr.v);
+    const bool plain = w.w == 0.0, ok = within<-200, 101>(l) & within<-200, 101>(r_);
+    const bool tl = nearer_zero(l, 1e-5), tr = nearer_zero(r_, 1e-5);
+    if (plain && ok) {
+        const xr s = half(l) + half(r_);
+        if (tl && tr) return xd(s.v);
+        const xr r = (tl ? xr(1e-5) : l) / (tr ? xr(1e-5) : r_);
+        if (xm::bits_of(r.v) >> 63) return xd(xm::double_of(xm::bits_of(s.v) & 0x8000000000000000ull));
+        const bool lt1 = below(r, 1.0);
+        xr phi = xr(2.0);
         bool quotient = true;
         if (lim == 1) {
             if (lt1) phi = twice(r);
         } else if (lt1) {
             quotient = false;
-            phi = lim == 0 ? (below(r, 0.5) ? twice(r) : xd(1.0)) : r;
+            phi = lim == 0 ? (below(r, 0.5) ? twice(r) : xr(1.0)) : r;
         }
-        if (quotient) phi = phi / (xd(1.0) + r);
-        return s * phi;
+        if (quotient) phi = phi / (xr(1.0) + r);
+        return xd((s * phi).v);
     }
+    const xd nan = xd(xm::double_of(0x7ff8000000000000ull));
+    if (!ok) return nan;
+    const xd s = (xd(w.a) * dl) + (xd(w.b) * dr);
+    const xd r = (tl ? xd(1e-5) : dl) / (tr ? xd(1e-5) : dr);
+    if (xm::plain_negative(r.v)) return xm::finite(s.v) ? xd(xm::double_of(xm::bits_of(s.v) & 0x8000000000000000ull)) : s;
+    if (!xm::plain_positive(r.v)) return nan;
+    const bool lt1 = below(r, 1.0);
     const xd xi = xd(2.0) / (xd(1.0 - w.w) + (xd(1.0 + w.w) * r));
     if (!xm::finite(xi.v)) return xi;  // a comparison would lose the NaN
     xd phi;
@@ -82,51 +91,89 @@ CG_D xd limited_slope(xd dl, xd dr, const Bias& w, int lim) {
     if (lim == 0 && 2.0 < phi.v) phi = xd(2.0);
     return s * phi;
 }
+// half of it, one copy for the integer pipes (300 instructions, five times per evolution)
+CG_D double half_slope(double dl, double dr, const Bias& w, int lim) { return half(limited_slope(dl, dr, w, lim)); }
+static __device__ __noinline__ xd half_slope(xd dl, xd dr, Bias w, int lim) { return half(limited_slope(dl, dr, w, lim)); }
 template <class T> CG_D void slope_exact(const T* ul, const T* uc, const T* ur, const Bias& w, int lim, T* s) {
 #pragma unroll
     for (int k = 0; k < 5; k++) s[k] = limited_slope(uc[k] - ul[k], ur[k] - uc[k], w, lim);
 }
 
+template <class T> CG_D V5<T> five(const T* a) { return V5<T>{{a[0], a[1], a[2], a[3], a[4]}}; }
+template <class T> CG_D void give(const V5<T>& a, T* o) {
+#pragma unroll
+    for (int k = 0; k < 5; k++) o[k] = a.v[k];
+}
+
 // ============================================================== Newtonian Euler
+// Velocities, two of their squares, specific total energy and pressure of a conserved state: what prim and
+// flux share.
+template <class T> struct NewtonParts { typename Raw<T>::type vx, vy, vz, xx, yy, et, pr; bool ok; };
+template <class T> CG_D NewtonParts<T> newton_parts(V5<T> in, double g1, bool fits) {
+    using R = typename Raw<T>::type;
+    R u[5];
+    NewtonParts<T> o;
+    o.ok = clean5(in.v, u) & fits;
+    const auto d = divisor(u[0]);
+    o.vx = u[1] / d;
+    o.vy = u[2] / d;
+    o.vz = u[3] / d;
+    o.et = u[4] / d;
+    o.xx = o.vx * o.vx;
+    o.yy = o.vy * o.vy;
+    const R v2 = (o.xx + o.yy) + (o.vz * o.vz);
+    o.pr = ((o.et - half(v2)) * R(g1)) * u[0];
+    return o;
+}
+
+// Bounds of the xr arithmetic, for inputs zero or in [2^-140, 2^100) (clean5), density not zero and
+// gamma - 1 in [2^-50, 2^50]: velocities in [2^-240, 2^240], their squares and products in [2^-480, 2^482],
+// a difference of such terms zero or at least one of their units, 2^-533; pressures in [2^-733, 2^633],
+// fluxes in [2^-973, 2^874].
 struct NewtonExact {
     double g, g1;  // gamma, gamma - 1
+    bool fits;     // gamma - 1 within the bounds
     static constexpr bool kCoords = false;
     NewtonExact() = default;
-    explicit NewtonExact(double gamma, int* = nullptr) : g(gamma), g1(gamma - 1.0) {}
+    explicit NewtonExact(double gamma, int* = nullptr)
+        : g(gamma), g1(gamma - 1.0), fits(gamma - 1.0 >= 0x1p-50 && gamma - 1.0 <= 0x1p50) {}
     // Euler/EulerStateVector.cpp:55-66, computeTotalEnergy :129-134, EoS Euler/EulerEquationOfState.cpp:3-8
-    template <class T> CG_D void cons(const T* p, Pt, T* u) const {
-        T rho = p[0], vx = p[1], vy = p[2], vz = p[3];
-        u[0] = rho; u[1] = rho * vx; u[2] = rho * vy; u[3] = rho * vz;
-        T v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
-        T e = p[4] / (T(g1) * rho);
-        u[4] = rho * (half(v2) + e);
+    template <class T> CG_D void cons(const T* in, Pt, T* u) const {
+        using R = typename Raw<T>::type;
+        R p[5];
+        const bool ok = clean5(in, p) & fits;
+        const R rho = p[0], vx = p[1], vy = p[2], vz = p[3];
+        const R v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
+        const R e = p[4] / (R(g1) * rho);
+        u[0] = given(rho, ok);
+        u[1] = given(rho * vx, true);
+        u[2] = given(rho * vy, true);
+        u[3] = given(rho * vz, true);
+        u[4] = given(rho * (half(v2) + e), true);
     }
     // Euler/EulerStateVector.cpp:30-40, computePressure Euler/EulerEquationOfState.cpp:10-15
     template <class T> CG_D void prim(const T* u, Pt, T* p) const {
-        T rho = u[0];
-        const auto d = divisor(rho);
-        T vx = u[1] / d, vy = u[2] / d, vz = u[3] / d;
-        T v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
-        T e = (u[4] / d) - half(v2);
-        p[0] = rho; p[1] = vx; p[2] = vy; p[3] = vz; p[4] = (e * T(g1)) * rho;
+        const NewtonParts<T> c = newton_parts(five(u), g1, fits);
+        using R = typename Raw<T>::type;
+        p[0] = given(R(u[0]), c.ok);
+        p[1] = given(c.vx, true);
+        p[2] = given(c.vy, true);
+        p[3] = given(c.vz, true);
+        p[4] = given(c.pr, true);
     }
     // Euler/EulerStateVector.cpp:68-89 (x) and :96-117 (y)
     template <class T> CG_D void flux(const T* u, int axis, Pt, T* f) const {
-        T rho = u[0];
-        const auto d = divisor(rho);
-        T vx = u[1] / d, vy = u[2] / d, vz = u[3] / d;
-        T xx = vx * vx, yy = vy * vy;
-        T v2 = (xx + yy) + (vz * vz);
-        T et = u[4] / d;
-        T pr = ((et - half(v2)) * T(g1)) * rho;
+        using R = typename Raw<T>::type;
+        const NewtonParts<T> c = newton_parts(five(u), g1, fits);
+        const R rho = R(u[0]);
         // products of two velocities commute exactly, so one form serves both axes
-        const T vn = axis == 0 ? vx : vy;
-        f[0] = rho * vn;
-        const T nn = (rho * (axis == 0 ? xx : yy)) + pr, xy = rho * (vx * vy);
-        f[1] = axis == 0 ? nn : xy;
-        f[2] = axis == 0 ? xy : nn;
-        f[3] = rho * (vn * vz);
-        f[4] = (rho * (vn * et)) + (vn * pr);
+        const R vn = axis == 0 ? c.vx : c.vy;
+        f[0] = given(rho * vn, c.ok);
+        const R nn = (rho * (axis == 0 ? c.xx : c.yy)) + c.pr, xy = rho * (c.vx * c.vy);
+        f[1] = given(axis == 0 ? nn : xy, true);
+        f[2] = given(axis == 0 ? xy : nn, true);
+        f[3] = given(rho * (vn * c.vz), true);
+        f[4] = given((rho * (vn * c.et)) + (vn * c.pr), true);
     }
     // Solvers/EulerSolvers.cpp:87-128 with Euler/EulerEquationOfState.cpp:17-22;
     // 2D is max(|vx|, |vy| + c) exactly as written at :117-118.
@@ -144,56 +191,79 @@ struct NewtonExact {
 // (:30-103, :159-350 with tol 1e-10 in the x flux at :205, :359-430).  Newton from x = 1 on the
 // quartic in x, stop when |x - x_new| < tol keeping the previous iterate, at most 1000 steps.
 template <class T> struct C2P { T rho, vx, vy, vz, p, W, h; };
+template <class T> CG_D void give_prim(const C2P<T>& c, T* p) {
+    p[0] = c.rho; p[1] = c.vx; p[2] = c.vy; p[3] = c.vz; p[4] = c.p;
+}
 // what the solve takes from gamma, formed once on the host
 struct GammaConst {
     double g, cst, lin, quad, gm, gm4, hg;
+    bool fits;  // gamma in [1 + 2^-50, 2^50]: the constants are zero or in [2^-101, 2^51]
     GammaConst() = default;
     // hg: gamma / (gamma - 1), the enthalpy's factor
     explicit GammaConst(double g_) : g(g_), cst(-1.0 / (g_ * g_)), lin((g_ - 1.0) / (g_ * g_)), quad((g_ - 2.0) / g_),
-                                     gm((g_ - 1.0) / g_), gm4(4.0 * ((g_ - 1.0) / g_)), hg(g_ / (g_ - 1.0)) {}
+                                     gm((g_ - 1.0) / g_), gm4(4.0 * ((g_ - 1.0) / g_)), hg(g_ / (g_ - 1.0)),
+                                     fits(g_ >= 1.0 + 0x1p-50 && g_ <= 0x1p50) {}
 };
 
 // One copy per number type (out of line): a sweep recovers eight states per cell, and the iteration
 // is thousands of cycles long.  status: ST_NEWTON_CAP is set there when the cap is reached (may be null).
+// Bounds of the xr arithmetic, for inputs zero or in [2^-140, 2^100): E in [2^-192, 2^101] (or zero), q
+// after its floor in [2^-27, 2^203], dc in [2^-242, 2^114], ec in [2^-295, 2^115], ec^2 in [2^-590, 2^230];
+// x in [2^-60, 2^60) at every iteration (tested), so that every term of f and fp lies within 2^-800 .. 2^580;
+// the step's quotient is an `xd` one; W in [2^-60, 2^60) (tested), so rho h W^2 lies within 2^-560 .. 2^640
+// and the velocities within 2^-780 .. 2^660.
+// (Two states in one instruction stream were 7 % slower on the relativistic sweeps: their code does not fit
+// the instruction caches.)
 template <class T>
-__device__ __noinline__ C2P<T> con2prim_exact(V5<T> u, GammaConst k, double tol, int* status) {
-    const T D = u.v[0], Sx = u.v[1], Sy = u.v[2], Sz = u.v[3], tau = u.v[4];
-    const T E = tau + D;
-    T q = (E * E) - (((Sx * Sx) + (Sy * Sy)) + (Sz * Sz));
+__device__ __noinline__ C2P<T> con2prim_exact(V5<T> in, GammaConst k, double tol, int* status) {
+    using R = typename Raw<T>::type;
+    R u[5];
+    bool ok = clean5(in.v, u) & k.fits;
+    const R D = u[0], Sx = u[1], Sy = u[2], Sz = u[3], tau = u[4];
+    const R E = tau + D;
+    const R q = (E * E) - (((Sx * Sx) + (Sy * Sy)) + (Sz * Sz));
     const bool tiny = below(q, 1e-8);
-    const auto dq = divisor(root(tiny ? T(1e-8) : q));
-    const T dc = D / dq, ec = E / dq;
-    const T ec2 = ec * ec;
-    const T linear = -(twice(dc) * T(k.lin));
-    const T quartic = ec2 - T(1.0);
-    const T quadratic = ((T(k.quad) * quartic) + T(1.0)) - (((dc * dc) * T(k.gm)) * T(k.gm));
-    const T eta = twice(dc) * T(k.gm);
-    const T quad2 = twice(quadratic), quart4 = fourfold(quartic), eta3 = (T(3.0) * eta) * quartic;
-    T x = T(1.0);
+    const auto dq = divisor(root(tiny ? R(1e-8) : q));
+    const R dc = D / dq, ec = E / dq;
+    const R ec2 = ec * ec;
+    const R linear = -(twice(dc) * R(k.lin));
+    const R quartic = ec2 - R(1.0);
+    const R quadratic = ((R(k.quad) * quartic) + R(1.0)) - (((dc * dc) * R(k.gm)) * R(k.gm));
+    const R eta = twice(dc) * R(k.gm);
+    const R quad2 = twice(quadratic), quart4 = fourfold(quartic), eta3 = (R(3.0) * eta) * quartic;
+    R x = R(1.0);
     int it = 0;
     bool conv = false;
-    while (it < 1000) {
-        const T x2 = x * x, x3 = x2 * x;
-        const T f = ((((quartic * x3) * (x - eta)) + (quadratic * x2)) + (linear * x)) + T(k.cst);
-        const T fp = ((linear + (quad2 * x)) + (quart4 * x3)) - (eta3 * x2);
-        const T nx = x - (f / fp);
+    while (it < 1000 && ok) {
+        const R x2 = x * x, x3 = x2 * x;
+        const R f = ((((quartic * x3) * (x - eta)) + (quadratic * x2)) + (linear * x)) + R(k.cst);
+        const R fp = ((linear + (quad2 * x)) + (quart4 * x3)) - (eta3 * x2);
+        const R nx = x - checked_quotient(f, fp);
         if (nearer_zero(x - nx, tol)) { conv = true; break; }
         it += 1;
         x = nx;
-        if (hopeless(nx)) return C2P<T>{nx, nx, nx, nx, nx, nx, nx};
+        ok = !hopeless(nx);
     }
-    if (!conv && status) atomicOr(status, ST_NEWTON_CAP);
+    if (!conv && ok && status) atomicOr(status, ST_NEWTON_CAP);
     C2P<T> r;
-    const T dx = dc * x;
-    r.W = (half(ec) * x) * (T(1.0) + root(T(1.0) + (T(k.gm4) * ((T(1.0) - dx) / (ec2 * (x * x))))));
-    r.h = T(1.0) / dx;
-    r.rho = D / r.W;
-    const T rhw = (r.rho * r.h) * (r.W * r.W);
+    const R dx = dc * x;
+    const R rt = root(R(1.0) + (R(k.gm4) * ((R(1.0) - dx) / (ec2 * (x * x)))));
+    const R W = (half(ec) * x) * (R(1.0) + rt);
+    ok = ok & within<-60, 60>(W);
+    const R h = R(1.0) / dx;
+    R rho = D / W;
+    const R rhw = (rho * h) * (W * W);
     const auto dr = divisor(rhw);
-    r.vx = Sx / dr; r.vy = Sy / dr; r.vz = Sz / dr;
-    r.p = (rhw - D) - tau;
-    if (below(r.rho, 1e-8)) r.rho = T(1e-8);
-    if (below(r.p, 1e-8)) r.p = T(1e-8);
+    R p = (rhw - D) - tau;
+    if (below(rho, 1e-8)) rho = R(1e-8);
+    if (below(p, 1e-8)) p = R(1e-8);
+    r.rho = given(rho, ok);
+    r.vx = given(Sx / dr, ok);
+    r.vy = given(Sy / dr, ok);
+    r.vz = given(Sz / dr, ok);
+    r.p = given(p, ok);
+    r.W = given(W, ok);
+    r.h = given(h, ok);
     return r;
 }
 
@@ -218,32 +288,44 @@ struct SRExact {
     static constexpr bool kCoords = false;
     SRExact() = default;
     explicit SRExact(double gamma, int* st = nullptr) : k(gamma), status(st) {}
-    // RelativisticEuler/RelativisticEulerStateVector.cpp:116-136
-    template <class T> CG_D void cons(const T* p, Pt, T* u) const {
-        T rho = p[0], vx = p[1], vy = p[2], vz = p[3], pr = p[4];
-        T v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
-        T W = lorentz(v2);
-        T h = sr_enthalpy(rho, pr, k);
-        T rhw = (rho * h) * (W * W);
-        u[0] = rho * W; u[1] = rhw * vx; u[2] = rhw * vy; u[3] = rhw * vz;
-        u[4] = (rhw - pr) - u[0];
+    // RelativisticEuler/RelativisticEulerStateVector.cpp:116-136.  Bounds: W in [1, 2^14], the enthalpy in
+    // [2^-53, 2^341] (p / rho within 2^-240 .. 2^240), rho h W^2 in [2^-193, 2^469].
+    template <class T> CG_D void cons(const T* in, Pt, T* u) const {
+        using R = typename Raw<T>::type;
+        R p[5];
+        const bool ok = clean5(in, p) & k.fits;
+        const R rho = p[0], vx = p[1], vy = p[2], vz = p[3], pr = p[4];
+        const R v2 = ((vx * vx) + (vy * vy)) + (vz * vz);
+        const R W = lorentz(v2);
+        const R h = sr_enthalpy(rho, pr, k);
+        const R rhw = (rho * h) * (W * W), D = rho * W;
+        u[0] = given(D, ok);
+        u[1] = given(rhw * vx, true);
+        u[2] = given(rhw * vy, true);
+        u[3] = given(rhw * vz, true);
+        u[4] = given((rhw - pr) - D, true);
     }
     template <class T> CG_D void prim(const T* u, Pt, T* p) const {
-        C2P<T> c = con2prim_exact(V5<T>{{u[0], u[1], u[2], u[3], u[4]}}, k, 1e-8, status);
-        p[0] = c.rho; p[1] = c.vx; p[2] = c.vy; p[3] = c.vz; p[4] = c.p;
+        give_prim(con2prim_exact(five(u), k, 1e-8, status), p);
     }
-    // RelativisticEuler/RelativisticEulerStateVector.cpp:138-220 (x), :227-309 (y)
+    // RelativisticEuler/RelativisticEulerStateVector.cpp:138-220 (x), :227-309 (y).  Bounds beyond the
+    // recovery's: velocities zero or in [2^-200, 2^100) (tested), so the terms lie within 2^-960 .. 2^840.
+    template <class T> CG_D void flux_of(const C2P<T>& c, int axis, T* f) const {
+        using R = typename Raw<T>::type;
+        const R rho = R(c.rho), vx = R(c.vx), vy = R(c.vy), vz = R(c.vz), p = R(c.p), W = R(c.W), h = R(c.h);
+        const bool ok = within<-60, 200>(rho) & within<-200, 100>(vx) & within<-200, 100>(vy) & within<-200, 100>(vz);
+        const R rhw = (rho * h) * (W * W);
+        const R vn = axis == 0 ? vx : vy;
+        const R rw = rho * W;
+        f[0] = given(rw * vn, ok);
+        const R nn = (rhw * (vn * vn)) + p, xy = rhw * (vx * vy);
+        f[1] = given(axis == 0 ? nn : xy, true);
+        f[2] = given(axis == 0 ? xy : nn, true);
+        f[3] = given(rhw * (vz * vn), true);
+        f[4] = given((((rhw - p) - rw) * vn) + (p * vn), true);
+    }
     template <class T> CG_D void flux(const T* u, int axis, Pt, T* f) const {
-        C2P<T> c = con2prim_exact(V5<T>{{u[0], u[1], u[2], u[3], u[4]}}, k, 1e-8, status);
-        T rhw = (c.rho * c.h) * (c.W * c.W);
-        T vn = axis == 0 ? c.vx : c.vy;
-        const T rw = c.rho * c.W;
-        f[0] = rw * vn;
-        const T nn = (rhw * (vn * vn)) + c.p, xy = rhw * (c.vx * c.vy);
-        f[1] = axis == 0 ? nn : xy;
-        f[2] = axis == 0 ? xy : nn;
-        f[3] = rhw * (c.vz * vn);
-        f[4] = (((rhw - c.p) - rw) * vn) + (c.p * vn);
+        flux_of(con2prim_exact(five(u), k, 1e-8, status), axis, f);
     }
     // Solvers/RelativisticEulerSolvers.cpp:87-128 (2D: max(|vx|, |vy|) + c)
     template <class T> CG_D T wavespeed(const T* p, int dims, Pt) const {
@@ -469,18 +551,19 @@ struct GRExact {
         for (int f = 0; f < 3; f++) u[1 + f] = srhw * p[1 + f];
         u[4] = g.sg * ((((p[0] * hh) * W) - p[4]) - (p[0] * W));
     }
-    template <class T> CG_D C2P<T> c2p(const T* u, T sg, double tol) const {
+    template <class T> CG_D V5<T> undensitised(const T* u, T sg) const {
         const auto d = divisor(sg);
-        return con2prim_exact(V5<T>{{u[0] / d, u[1] / d, u[2] / d, u[3] / d, u[4] / d}}, k, tol, status);
+        return V5<T>{{u[0] / d, u[1] / d, u[2] / d, u[3] / d, u[4] / d}};
+    }
+    template <class T> CG_D C2P<T> c2p(const T* u, T sg, double tol) const {
+        return con2prim_exact(undensitised(u, sg), k, tol, status);
     }
     // BlackHoleEuler/BlackHoleEulerStateVector.cpp:30-103
     template <class T> CG_D void prim_in(const Metric<T>& g, const T* u, T* p) const {
-        C2P<T> c = c2p(u, g.sg, 1e-8);
-        p[0] = c.rho; p[1] = c.vx; p[2] = c.vy; p[3] = c.vz; p[4] = c.p;
+        give_prim(c2p(u, g.sg, 1e-8), p);
     }
     // BlackHoleEuler/BlackHoleEulerStateVector.cpp:159-250 (x, tol 1e-10) and :259-350 (y)
-    template <class T> CG_D void flux_in(const Metric<T>& g, const T* u, int axis, T* f) const {
-        C2P<T> c = c2p(u, g.sg, axis == 0 ? 1e-10 : 1e-8);
+    template <class T> CG_D void flux_of(const Metric<T>& g, const C2P<T>& c, int axis, T* f) const {
         const T as = g.al * g.sg;
         const T rhw = (c.rho * c.h) * (c.W * c.W);
         const T vn = axis == 0 ? c.vx : c.vy;
@@ -492,6 +575,9 @@ struct GRExact {
         f[2] = as * (axis == 0 ? y : y + c.p);
         f[3] = as * (rhw * (c.vz * w));
         f[4] = as * ((((rhw - c.p) - rw) * w) + (c.p * vn));
+    }
+    template <class T> CG_D void flux_in(const Metric<T>& g, const T* u, int axis, T* f) const {
+        flux_of(g, c2p(u, g.sg, axis == 0 ? 1e-10 : 1e-8), axis, f);
     }
     // ---- metric derivatives (BlackHoleSpacetime.cpp:115-151, :250-334), centred with spacing h
     CG_D Pt off(Pt q, int d, double s) const {
@@ -661,11 +747,6 @@ __device__ __noinline__ V5<T> gr_source(const GRExact* S, const Metric<T>* g, co
     S->source_in(*g, *sm, u.v, o.v);
     return o;
 }
-template <class T> CG_D V5<T> five(const T* a) { return V5<T>{{a[0], a[1], a[2], a[3], a[4]}}; }
-template <class T> CG_D void give(const V5<T>& a, T* o) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) o[k] = a.v[k];
-}
 template <class T> CG_D void GRExact::cons(const T* p, Pt q, T* u) const {
     Metric<T> g;
     gr_metric(this, q, &g);
@@ -690,6 +771,10 @@ template <class T> CG_D void GRExact::source(const T* u, Pt q, T* s) const {
 }
 
 // ============================================================== generic evolution pieces
+// The sums of the stages: half (a + c b), and a + c b.
+template <class T> CG_D T half_mix(T a, T b, T c) { return half(a + (c * b)); }
+template <class T> CG_D T plus_times(T a, T b, T c) { return a + (c * b); }
+
 // Half-step evolution (Solvers/EulerSolvers.cpp:174-223; SR Solvers/RelativisticEulerSolvers.cpp:148-199;
 // GR Solvers/BlackHoleEulerSolvers.cpp:234-307) from the conserved states of the cell and its two
 // neighbours.  Produces the left- and/or right-face state as primitives (the reference's evolved
@@ -700,12 +785,13 @@ CG_D void evolve_half_cons(const Sys& S, const T* ul, const T* um, const T* ur, 
     T UL[5], UR[5], FL[5], FR[5];
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        const T hs = half(limited_slope(um[k] - ul[k], ur[k] - um[k], w, lim));
+        const T hs = half_slope(um[k] - ul[k], ur[k] - um[k], w, lim);
         UL[k] = um[k] - hs;
         UR[k] = um[k] + hs;
     }
-    S.flux(UL, axis, shift_pt(xc, axis, -(dx * 0.5)), FL);
-    S.flux(UR, axis, shift_pt(xc, axis, dx * 0.5), FR);
+    const Pt pl = shift_pt(xc, axis, -(dx * 0.5)), pr = shift_pt(xc, axis, dx * 0.5);
+    S.flux(UL, axis, pl, FL);
+    S.flux(UR, axis, pr, FR);
     const T s = half(T(st.d));
 #pragma unroll
     for (int k = 0; k < 5; k++) {
@@ -713,8 +799,8 @@ CG_D void evolve_half_cons(const Sys& S, const T* ul, const T* um, const T* ur, 
         UL[k] = UL[k] + ev;
         UR[k] = UR[k] + ev;
     }
-    if (left_face) S.prim(UL, shift_pt(xc, axis, -(dx * 0.5)), left_face);
-    if (right_face) S.prim(UR, shift_pt(xc, axis, dx * 0.5), right_face);
+    if (left_face) S.prim(UL, pl, left_face);
+    if (right_face) S.prim(UR, pr, right_face);
 }
 // ... from their primitive states
 template <class Sys, class T>
@@ -737,8 +823,8 @@ CG_D void force_cons(const Sys& S, const T* uL, const T* uR, Pt xf, int axis, do
     const T c = T(st.c), d = T(st.d);
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        us[k] = half((uL[k] + uR[k]) + (d * (fL[k] - fR[k])));
-        F[k] = half((fL[k] + fR[k]) + (c * (uL[k] - uR[k])));
+        us[k] = half_mix(uL[k] + uR[k], fL[k] - fR[k], d);
+        F[k] = half_mix(fL[k] + fR[k], uL[k] - uR[k], c);
     }
     S.flux(us, axis, xf, fs);
 #pragma unroll
@@ -770,30 +856,31 @@ CG_D void gr_interface(const GRExact* S, const V5<T>* c, int order, Pt xf, int a
         gr_metric(S, xc, &gc);
         V5<T> face = c[1 + side];
         if (order == 2) {
-            Metric<T> gm;
+            Metric<T> go;
             const V5<T> um = gr_cons(S, &gc, c[1 + side]);
-            gr_metric(S, shift_pt(xc, axis, -dx), &gm);
-            const V5<T> ul = gr_cons(S, &gm, c[side]);
-            gr_metric(S, shift_pt(xc, axis, dx), &gm);
-            const V5<T> ur = gr_cons(S, &gm, c[2 + side]);
+            gr_metric(S, shift_pt(xc, axis, -dx), &go);
+            const V5<T> ul = gr_cons(S, &go, c[side]);
+            gr_metric(S, shift_pt(xc, axis, dx), &go);
+            const V5<T> ur = gr_cons(S, &go, c[2 + side]);
             V5<T> UL, UR;
 #pragma unroll
             for (int k = 0; k < 5; k++) {
-                const T hs = half(limited_slope(um.v[k] - ul.v[k], ur.v[k] - um.v[k], w, lim));
+                const T hs = half_slope(um.v[k] - ul.v[k], ur.v[k] - um.v[k], w, lim);
                 UL.v[k] = um.v[k] - hs;
                 UR.v[k] = um.v[k] + hs;
             }
-            // the face wanted lies at xc + dx/2 (left cell) or xc - dx/2 (right cell): its point last
+            // the face wanted lies at xc + dx/2 (left cell) or xc - dx/2 (right cell)
             const T s = half(T(st.d));
-            gr_metric(S, shift_pt(xc, axis, side == 0 ? -(dx * 0.5) : dx * 0.5), &gm);
-            const V5<T> fo = gr_flux(S, &gm, side == 0 ? UL : UR, axis);
-            gr_metric(S, shift_pt(xc, axis, side == 0 ? dx * 0.5 : -(dx * 0.5)), &gm);
-            V5<T> U = side == 0 ? UR : UL;
-            const V5<T> fi = gr_flux(S, &gm, U, axis);
+            gr_metric(S, shift_pt(xc, axis, side == 0 ? -(dx * 0.5) : dx * 0.5), &go);
+            const V5<T> V = side == 0 ? UL : UR;
+            V5<T> X = side == 0 ? UR : UL;
+            const V5<T> fo = gr_flux(S, &go, V, axis);
+            gr_metric(S, shift_pt(xc, axis, side == 0 ? dx * 0.5 : -(dx * 0.5)), &go);
+            const V5<T> fi = gr_flux(S, &go, X, axis);
 #pragma unroll
             for (int k = 0; k < 5; k++)
-                U.v[k] = U.v[k] + (s * (side == 0 ? fo.v[k] - fi.v[k] : fi.v[k] - fo.v[k]));
-            face = gr_prim(S, &gm, U);
+                X.v[k] = X.v[k] + (s * (side == 0 ? fo.v[k] - fi.v[k] : fi.v[k] - fo.v[k]));
+            face = gr_prim(S, &go, X);
         }
         uf[side] = gr_cons(S, &gc, face);
         ff[side] = gr_flux(S, &gc, uf[side], axis);
@@ -802,8 +889,8 @@ CG_D void gr_interface(const GRExact* S, const V5<T>* c, int order, Pt xf, int a
     const T cc = T(st.c), d = T(st.d);
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        us.v[k] = half((uf[0].v[k] + uf[1].v[k]) + (d * (ff[0].v[k] - ff[1].v[k])));
-        F[k] = half((ff[0].v[k] + ff[1].v[k]) + (cc * (uf[0].v[k] - uf[1].v[k])));
+        us.v[k] = half_mix(uf[0].v[k] + uf[1].v[k], ff[0].v[k] - ff[1].v[k], d);
+        F[k] = half_mix(ff[0].v[k] + ff[1].v[k], uf[0].v[k] - uf[1].v[k], cc);
     }
     gr_metric(S, xf, &gc);
     const V5<T> fs = gr_flux(S, &gc, us, axis);
@@ -833,7 +920,7 @@ CG_D V5<T> evolve_fraction_in(const GRExact* S, double frac, const V5<T>& ul, co
     V5<T> um = gr_cons(S, gm, m), UL, UR;
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        const T hs = half(limited_slope(um.v[k] - ul.v[k], ur.v[k] - um.v[k], w, lim));
+        const T hs = half_slope(um.v[k] - ul.v[k], ur.v[k] - um.v[k], w, lim);
         UL.v[k] = um.v[k] - hs;
         UR.v[k] = um.v[k] + hs;
     }
