@@ -128,12 +128,20 @@ bool valid_params(const cosmos_params* p, std::string& why) {
 // [GR: subcycles RK source half-steps], and the CFL reduction for the next step.
 int enqueue_step(cosmos_grid* g, int cur, int* cur_out, unsigned* nk) {
     const cosmos_solve_opts& o = g->run;
-    CK(launch_dt_kernel(g->ctl, g->ctx->stream));
-    unsigned k = 1;
     SweepArgs a = base_args(g);
     a.order = o.order;
     a.bias = o.bias;
     a.lim = o.limiter;
+    if (g->p.precision == COSMOS_FP32 && fused_step_fast(g->G, g->p.system, o.order)) {
+        a.src = g->buf[cur];
+        a.dst = g->buf[cur ^ 1];
+        CK(launch_fused_step_fast(a, g->ctl));
+        *nk = 1;
+        *cur_out = cur ^ 1;
+        return COSMOS_OK;
+    }
+    CK(launch_dt_kernel(g->ctl, g->ctx->stream));
+    unsigned k = 1;
     a.out.status = &g->ctl->status;
     a.ds.ctl = g->ctl;
     auto sweep = [&](int axis, double scale, bool ws) -> int {

@@ -72,6 +72,7 @@ struct StepCtl {
     StepRatio xr[2];   // the same ratios in FP64
     double* dt_log;           // non-null: the dt kernel records each step's dt at dt_log[it]
     const double* dt_fixed;   // non-null: step `it` takes dt_fixed[it] instead of the CFL rule
+    unsigned int done;        // fused steps (step_tile.cuh): blocks that have finished, 0 between launches
 };
 
 // Status bits written by kernels (mirrored in include/cosmos_gb300.h)
@@ -88,40 +89,60 @@ enum : int {
 // its latency counts: five FP64 divisions of 565 cycles each one after the other were 1.4 us; the
 // quotients come from the integer pipes (three of about 240 cycles, two of them independent), and
 // those of dt/2 are the ones of dt halved and doubled, which is exact.
-CG_D void step_ctl_advance(StepCtl* c) {
+struct StepNow {
+    bool active;
+    double dt;
+    StepRatio r, h;  // dt / dx and dx / dt, for dt and for dt / 2
+    CG_D FastCoef full() const { return FastCoef{(float)r.d, (float)(0.5 * r.d), (float)(0.25 * r.c)}; }
+    CG_D FastCoef halved() const { return FastCoef{(float)h.d, (float)(0.5 * h.d), (float)(0.25 * h.c)}; }
+};
+CG_D StepNow step_now(const StepCtl* c) {
+    StepNow s;
     const double t = c->t, t_final = c->t_final, dx = c->dx;
     const int it = c->it;
-    if (!(t < t_final) || it >= c->it_limit) {
+    s.active = t < t_final && it < c->it_limit;
+    s.dt = 0.0;
+    s.r = s.h = StepRatio{0.0, 0.0};
+    if (!s.active) return s;
+    if (c->dt_fixed) {
+        s.dt = c->dt_fixed[it];
+    } else {
+        const unsigned long long m0 = c->smax[0], m1 = c->smax[1];  // both, so that no load waits for `it`
+        const double smax = __longlong_as_double((long long)(it & 1 ? m1 : m0));
+        s.dt = c->cfl * quotient(dx, smax);
+        if (it <= 5) s.dt = s.dt * 0.2;
+        if ((t + s.dt) > t_final) s.dt = t_final - t;
+    }
+    s.r = StepRatio{xm::div(s.dt, dx), xm::div(dx, s.dt)};
+    s.h = StepRatio{0.5 * s.r.d, 2.0 * s.r.c};
+    if (!xm::finite(s.r.d + s.r.c)) {
+        s.r = make_ratio(s.dt, dx);
+        s.h = make_ratio(s.dt * 0.5, dx);
+    }
+    return s;
+}
+// Enters the step into the controller; `clear` is the CFL slot emptied for a later reduction.
+CG_D void step_enter(StepCtl* c, const StepNow& s, int clear) {
+    const int it = c->it;
+    if (!s.active) {
         c->active = 0;
         c->dt = 0.0;
         return;
     }
-    double dt;
-    if (c->dt_fixed) {
-        dt = c->dt_fixed[it];
-    } else {
-        const double smax = __longlong_as_double((long long)c->smax[it & 1]);
-        dt = c->cfl * quotient(dx, smax);
-        if (it <= 5) dt = dt * 0.2;
-        if ((t + dt) > t_final) dt = t_final - t;
-    }
-    if (!(dt > 0.0) || !isfinite(dt)) c->status |= ST_NONFINITE;
-    if (c->dt_log) c->dt_log[it] = dt;
-    c->dt = dt;
-    StepRatio r{xm::div(dt, dx), xm::div(dx, dt)}, h{0.5 * r.d, 2.0 * r.c};
-    if (!xm::finite(r.d + r.c)) {
-        r = make_ratio(dt, dx);
-        h = make_ratio(dt * 0.5, dx);
-    }
-    c->xr[0] = r;
-    c->xr[1] = h;
-    c->fc[0] = FastCoef{(float)r.d, (float)(0.5 * r.d), (float)(0.25 * r.c)};
-    c->fc[1] = FastCoef{(float)h.d, (float)(0.5 * h.d), (float)(0.25 * h.c)};
+    if (!(s.dt > 0.0) || !isfinite(s.dt)) c->status |= ST_NONFINITE;
+    if (c->dt_log) c->dt_log[it] = s.dt;
+    c->dt = s.dt;
+    c->xr[0] = s.r;
+    c->xr[1] = s.h;
+    c->fc[0] = s.full();
+    c->fc[1] = s.halved();
     c->active = 1;
-    c->smax[(it + 1) & 1] = 0ull;
-    c->t = t + dt;
+    c->smax[clear] = 0ull;
+    c->t = c->t + s.dt;
     c->it = it + 1;
 }
+// before a step's sweeps: they reduce into the other slot, emptied here
+CG_D void step_ctl_advance(StepCtl* c) { step_enter(c, step_now(c), (c->it + 1) & 1); }
 
 // Max of non-negative doubles (ordering of their bit patterns equals numeric ordering).
 // The slot only grows while a kernel reduces into it, so a block whose value does not exceed what

@@ -5,6 +5,7 @@
 
 #include "launch.h"
 #include "policies.cuh"
+#include "step_tile.cuh"
 #include "sweep_pairs.cuh"
 
 namespace cg {
@@ -68,6 +69,10 @@ bool field_map(CUtensorMap* m, const float* base, const Geom& G, unsigned box_x)
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+
+// us per step, three sweeps against one launch (MinBee): 50x60 15.6 / 10.9, 193x257 18.3 / 10.9, 400^2 19.9 /
+// 13.9, 512^2 21.8 / 19.9, 640^2 26.4 / 27.2, 1024^2 43.1 / 54.1.
+constexpr size_t kFusedStepCells = 300000;
 
 namespace {
 
@@ -213,6 +218,33 @@ cudaError_t launch_prim_out_fast(const void* soa, double* aos, const Geom& G, in
     prim_out_fast_kernel<<<grid_for((size_t)G.nx * G.ny), 256, 0, st>>>((const float*)soa, aos, G, gamma);
     count_launch();
     return cudaGetLastError();
+}
+
+// Whole steps in one launch: two-dimensional SLIC without a mask, up to kFusedStepCells cells.
+bool fused_step_fast(const Geom& G, int system, int order) {
+    return system == 0 && order == 2 && G.dims == 2 && G.nx >= 8 && G.ny >= 8 && (size_t)G.nx * G.ny <= kFusedStepCells;
+}
+
+namespace {
+template <int LIM>
+cudaError_t run_fused(const SweepArgs& a, StepCtl* ctl) {
+    const Geom& G = a.G;
+    const auto P = make_newton_fast<0, LIM, false>(a.gamma, a.bias, G.nx, G.dims).P;
+    const cudaError_t e = cudaFuncSetAttribute(step_tile_kernel<LIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(StepTileSmem));
+    if (e != cudaSuccess) return e;
+    const dim3 grid((G.nx + kTileCols - 1) / kTileCols, (G.ny + kTileRows - 1) / kTileRows);
+    step_tile_kernel<LIM><<<grid, kTileWarps * 32, sizeof(StepTileSmem), a.stream>>>(P, G, (const float*)a.src,
+                                                                                     (float*)a.dst, ctl);
+    count_launch();
+    return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_fused_step_fast(const SweepArgs& a, StepCtl* ctl) {
+    if (a.lim == 0) return run_fused<0>(a, ctl);
+    if (a.lim == 1) return run_fused<1>(a, ctl);
+    return run_fused<2>(a, ctl);
 }
 
 }  // namespace cg

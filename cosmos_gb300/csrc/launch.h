@@ -116,6 +116,10 @@ cudaError_t launch_sweep_fast(const SweepArgs& a);
 // five fields G.fstride apart) whose box is `box_x` cells of one row in every field; false when
 // the state cannot be described (the sweeps then copy each field by itself).
 bool field_map(CUtensorMap_st* m, const float* base, const Geom& G, unsigned box_x);
+// One whole step of an FP32 Newtonian SLIC run (its time step, X Y X, CFL reduction) in one launch, for the
+// grids fused_step_fast accepts; a.src to a.dst, the controller entered by the launch itself.
+bool fused_step_fast(const Geom& G, int system, int order);
+cudaError_t launch_fused_step_fast(const SweepArgs& a, StepCtl* ctl);
 cudaError_t launch_wavespeed_fast(const SweepArgs& a, unsigned long long* slot);
 cudaError_t launch_prim_in_fast(const double* aos, void* soa, const Geom& G, int system, double gamma,
                                 cudaStream_t st);
