@@ -22,24 +22,6 @@ constexpr int kYPairThreads = 32;  // one warp (64 columns, two per thread) per 
 constexpr int kYRingRows = 8;      // Y rows staged in shared memory per warp (up to 8 in flight)
 constexpr int kYRingMinBlocks = 16;  // at most 128 registers: 16 one-warp blocks per SM
 
-// Rows per Y-sweep block: about 32 (each block re-reads four halo rows), adjusted so that the
-// blocks fill whole waves of the resident slots.  At 4096^2, 32-row segments make 8192 one-warp
-// blocks for 152 x 16 slots (3.37 waves, the last a third full); 36-row segments make 7296, three
-// full waves.
-int y_ring_seg(const void* kernel, int nx, int ny) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kYPairThreads, 0) != cudaSuccess || per_sm < 1)
-        per_sm = kYRingMinBlocks;
-    const long long slots = (long long)per_sm * device_sm_count();
-    const long long cols = (nx + 2 * kYPairThreads - 1) / (2 * kYPairThreads);
-    const long long blocks32 = cols * ((ny + 31) / 32);
-    const long long waves = blocks32 / slots > 1 ? blocks32 / slots : 1;
-    long long rows = waves * slots / cols;  // block rows that fill `waves` whole waves
-    if (rows < 1) rows = 1;
-    int seg = (int)((ny + rows - 1) / rows);
-    return seg < 8 ? 8 : (seg > 64 ? 64 : seg);
-}
-
 // cuTensorMapEncodeTiled through the runtime's driver entry point (nullptr when the driver does
 // not provide it).
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -57,6 +39,19 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 }  // namespace
 
 std::atomic<int> g_tensor_maps{1};
+
+int wave_rows(const void* kernel, int threads, int cols_per_block, int nx, int ny, int about) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1) per_sm = 16;
+    const long long slots = (long long)per_sm * device_sm_count();
+    const long long cols = (nx + cols_per_block - 1) / cols_per_block;
+    const long long blocks = cols * ((ny + about - 1) / about);
+    const long long waves = blocks / slots > 1 ? blocks / slots : 1;
+    long long rows = waves * slots / cols;  // block rows that fill `waves` whole waves
+    if (rows < 1) rows = 1;
+    const int seg = (int)((ny + rows - 1) / rows);
+    return seg < 8 ? 8 : (seg > 64 ? 64 : seg);
+}
 
 bool field_map(CUtensorMap* m, const float* base, const Geom& G, unsigned box_x) {
     if (!g_tensor_maps.load(std::memory_order_relaxed)) return false;
@@ -112,14 +107,14 @@ cudaError_t run_fast(const SweepArgs& a) {
         const bool use_tm = field_map(&tm, src, G, 64);  // 4096^2: 0.136 ms against 0.150 with per-field copies
         auto kernel = use_tm ? sweep_y_ring_kernel<LIM, kYPairThreads, kYRingRows, kYRingMinBlocks, true>
                              : sweep_y_ring_kernel<LIM, kYPairThreads, kYRingRows, kYRingMinBlocks, false>;
-        const int seg = y_ring_seg((const void*)kernel, G.nx, G.ny);
+        const int seg = wave_rows((const void*)kernel, kYPairThreads, 2 * kYPairThreads, G.nx, G.ny, 32);
         dim3 grid((G.nx + 2 * kYPairThreads - 1) / (2 * kYPairThreads), (G.ny + seg - 1) / seg);
         kernel<<<grid, kYPairThreads, 0, a.stream>>>(pol.P, G.dims, G, src, dst, a.ds, a.out, seg, tm);
         return cudaSuccess;
     } else {
         dim3 grid((G.nx + kYThreads - 1) / kYThreads, (G.ny + kYSeg - 1) / kYSeg);
-        if (a.order == 2) sweep_y_kernel<Pol, 2, kYThreads, kYSeg><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
-        else sweep_y_kernel<Pol, 1, kYThreads, kYSeg><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
+        if (a.order == 2) sweep_y_kernel<Pol, 2, kYThreads><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out, kYSeg);
+        else sweep_y_kernel<Pol, 1, kYThreads><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out, kYSeg);
     }
     return cudaSuccess;
 }

@@ -198,14 +198,13 @@ GRFastPolicy<AXIS, LIM, MASKED> make_pol(const SweepArgs& a, double bias) {
     return p;
 }
 
-constexpr int kXThreads = 256;
-// One warp of columns per Y block, 8 rows per segment: the cells near the hole (FP64 recovery
+constexpr int kXThreads = 64;  // 62 updates per tile; 1024^2, 6 steps: 256 threads 1389 us per step, 128 1372, 64 1363, 32 1375
+// One warp of columns per Y block, 4 rows per segment: the cells near the hole (FP64 recovery
 // stage) make some column segments several times costlier than the rest, and many small blocks
-// spread them over the SMs (at 1024^2, 4096 blocks of 32 x 8 cells against 256 of 128 x 32; the
-// 4-row halo of each segment costs less than the imbalance it removes: 2.49 vs 2.65 ms per step
-// against 32 x 16).
+// spread them over the SMs; a small grid has more warps too.  us per step with 4 / 8 / 16 rows: 400^2 from rest
+// 248 / 261 / 295, 60 steps 661 / 722 / 820; 1024^2 from rest 1190 / 1173 / 1228, 60 steps 1380 / 1483 / 1537.
 constexpr int kYThreads = 32;
-constexpr int kYSeg = 8;
+constexpr int kYSeg = 4;
 
 template <int AXIS, int LIM, bool MASKED>
 void run(const SweepArgs& a) {
@@ -220,8 +219,8 @@ void run(const SweepArgs& a) {
         else sweep_x_own_kernel<Pol, 1, kXThreads><<<grid, kXThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
     } else {
         dim3 grid((G.nx + kYThreads - 1) / kYThreads, (G.ny + kYSeg - 1) / kYSeg);
-        if (a.order == 2) sweep_y_kernel<Pol, 2, kYThreads, kYSeg><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
-        else sweep_y_kernel<Pol, 1, kYThreads, kYSeg><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
+        if (a.order == 2) sweep_y_kernel<Pol, 2, kYThreads><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out, kYSeg);
+        else sweep_y_kernel<Pol, 1, kYThreads><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out, kYSeg);
     }
 }
 
@@ -234,10 +233,14 @@ void run_lim(const SweepArgs& a) {
 
 // ---------------------------------------------------------------- source step
 // One cell per thread; cells whose five-point stencil touches the excised region keep their state.
-// Capped at three blocks of 128 threads per SM (168 registers, a small L1-resident spill): on the
-// evolved 1024^2 accretion grid that beat 205 registers at two blocks (2.65 vs 2.81 ms per step).
-template <int LIM>
-__global__ void __launch_bounds__(128, 3) gr_rk_kernel(SRFastParams P, NewtonFastParams NP, GRTables T, Geom G, double dx,
+// Bound by instruction issue and by waiting for instructions (1.1 of 4.6 cycles with every recovery inlined at its
+// place), so the three fractional sweeps of a stage and the four stages' source terms share one copy of the code
+// each, and the neighbours' conserved states are formed once: 1024^2 steps 1363 -> 1211 us (6 steps from rest),
+// 1760 -> 1507 (60 steps).  Sharing the neighbours' recoveries too measured 1241 us.  384 threads per SM (168
+// registers): 256 1400 us, 512 1410.  Blocks of 64 threads, of 32 on small grids (400^2: 128 threads 261 us per
+// step, 64 251, 32 228; 1024^2: 1173, 1177, 1187).
+template <int LIM, int NT>
+__global__ void __launch_bounds__(NT, 384 / NT) gr_rk_kernel(SRFastParams P, NewtonFastParams NP, GRTables T, Geom G, double dx,
                                                     const float* __restrict__ src, float* __restrict__ dst, DtSrc ds,
                                                     int* status) {
     // the step's dt (0.5 dt / subcycles from the controller) and dt/dx, once per block
@@ -274,26 +277,26 @@ __global__ void __launch_bounds__(128, 3) gr_rk_kernel(SRFastParams P, NewtonFas
     // primitives of the cell and its neighbours, made conserved at their own centres
     // (the reference's kernel, Solvers/BlackHoleEulerForcingSolver.cpp:72-99)
     const int ii = G.dims == 1 ? 0 : i;
+    int flags = 0;
     const GRMet Ml = met(ii, j - 1), Mc = met(ii, j), Mr = met(ii, j + 1);
     GRMet Mt = Mc, Mb = Mc;
     float p[5], cl[5], cm[5], cr[5], ct[5], cb[5], out[5];
     ld(i, j - 1, p);
-    gr_cons_fast(P, p, Ml, cl);
-    ld(i, j, p);
-    gr_cons_fast(P, p, Mc, cm);
+    gr_frozen_fast(P, p, Ml, cl, &flags);
     ld(i, j + 1, p);
-    gr_cons_fast(P, p, Mr, cr);
+    gr_frozen_fast(P, p, Mr, cr, &flags);
     if (G.dims == 2) {
         Mt = met(i - 1, j);
         Mb = met(i + 1, j);
         ld(i - 1, j, p);
-        gr_cons_fast(P, p, Mt, ct);
+        gr_frozen_fast(P, p, Mt, ct, &flags);
         ld(i + 1, j, p);
-        gr_cons_fast(P, p, Mb, cb);
+        gr_frozen_fast(P, p, Mb, cb, &flags);
     }
+    ld(i, j, p);
+    gr_cons_fast(P, p, Mc, cm);
     GRSrc X;
     load_src(GRTab{T.src, T.cell_stride}, (size_t)i * G.nx + j, X);
-    int flags = 0;
     gr_rk_fast<LIM>(P, NP, G.dims, cl, cm, cr, ct, cb, Ml, Mc, Mr, Mt, Mb, X, s_dt, dtdx, out, &flags);
 #pragma unroll
     for (int f = 0; f < 5; f++) dst[f * G.fstride + idx] = out[f];
@@ -380,9 +383,12 @@ cudaError_t launch_sweep_gr_fast(const SweepArgs& a) {
 
 cudaError_t launch_rk_source_gr_fast(const SweepArgs& a) {
     const SRFastPolicy<0, 1, false> s = make_sr_fast<0, 1, false>(a.gamma, a.bias, a.G.nx, a.G.dims, a.c2p64_above);
-    dim3 grid((a.G.nx + 127) / 128, a.G.ny);
-    auto k = a.lim == 0 ? gr_rk_kernel<0> : (a.lim == 1 ? gr_rk_kernel<1> : gr_rk_kernel<2>);
-    k<<<grid, 128, 0, a.stream>>>(s.P, s.NP, *a.grt, a.G, a.dx, (const float*)a.src, (float*)a.dst, a.ds, a.out.status);
+    const bool small = (size_t)a.G.nx * a.G.ny < (size_t)1 << 19;
+    const int nt = small ? 32 : 64;
+    dim3 grid((a.G.nx + nt - 1) / nt, a.G.ny);
+    auto k = small ? (a.lim == 0 ? gr_rk_kernel<0, 32> : (a.lim == 1 ? gr_rk_kernel<1, 32> : gr_rk_kernel<2, 32>))
+                   : (a.lim == 0 ? gr_rk_kernel<0, 64> : (a.lim == 1 ? gr_rk_kernel<1, 64> : gr_rk_kernel<2, 64>));
+    k<<<grid, nt, 0, a.stream>>>(s.P, s.NP, *a.grt, a.G, a.dx, (const float*)a.src, (float*)a.dst, a.ds, a.out.status);
     count_launch();
     return cudaGetLastError();
 }

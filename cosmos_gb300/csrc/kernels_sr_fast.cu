@@ -7,9 +7,12 @@ namespace cg {
 
 namespace {
 
-constexpr int kXThreads = 256;
-constexpr int kYThreads = 128;
-constexpr int kYSeg = 32;
+// us per step of 2048^2 Kelvin-Helmholtz by X tile: 256 threads 609 (a row's ninth tile holds 16 cells), 128 568,
+// 64 577, 32 621.
+constexpr int kXThreads = 128;
+// One-warp Y blocks whose rows fill whole waves: 128-thread blocks of 32 rows were 1.68 waves at 2048^2 (643 ->
+// 609 us per step) and 64 blocks of them at 512^2 left most SMs idle (117 -> 68).
+constexpr int kYThreads = 32;
 
 template <int AXIS, int LIM, bool MASKED>
 SRFastPolicy<AXIS, LIM, MASKED> make_pol(const SweepArgs& a) {
@@ -28,9 +31,10 @@ void run(const SweepArgs& a) {
         if (a.order == 2) sweep_x_own_kernel<Pol, 2, kXThreads><<<grid, kXThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
         else sweep_x_own_kernel<Pol, 1, kXThreads><<<grid, kXThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
     } else {
-        dim3 grid((G.nx + kYThreads - 1) / kYThreads, (G.ny + kYSeg - 1) / kYSeg);
-        if (a.order == 2) sweep_y_kernel<Pol, 2, kYThreads, kYSeg><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
-        else sweep_y_kernel<Pol, 1, kYThreads, kYSeg><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
+        const auto kernel = a.order == 2 ? sweep_y_kernel<Pol, 2, kYThreads> : sweep_y_kernel<Pol, 1, kYThreads>;
+        const int seg = wave_rows((const void*)kernel, kYThreads, kYThreads, G.nx, G.ny, 32);
+        dim3 grid((G.nx + kYThreads - 1) / kYThreads, (G.ny + seg - 1) / seg);
+        kernel<<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out, seg);
     }
 }
 

@@ -110,6 +110,12 @@ cudaError_t launch_interface_eval(const SweepArgs& s, const IfaceArgs& a);
 constexpr int kSpacetimeWidth = 125;
 cudaError_t launch_spacetime_eval(const SweepArgs& s, size_t n, const double* xyz, double* out);
 
+// Rows per block of a marching Y sweep: about `about` (each block reads four halo rows again), adjusted so
+// that the blocks fill whole waves of the resident slots, 8 to 64.  At 4096^2, 32-row segments of the FP32
+// Newtonian sweep make 8192 one-warp blocks for 152 x 16 slots (3.37 waves, the last a third full); 36-row
+// segments make 7296, three full waves.
+int wave_rows(const void* kernel, int threads, int cols_per_block, int nx, int ny, int about);
+
 // FP32 bulk path (conserved SoA storage, float)
 cudaError_t launch_sweep_fast(const SweepArgs& a);
 // A 3-D tensor map of an FP32 SoA state at `base` (x: nx cells, y: ny rows G.pitch apart, z: the

@@ -81,7 +81,7 @@ CG_D SRPrim32 gr_c2p_fast(const SRFastParams& P, const float* u, const GRMet& M,
     float v[5];
 #pragma unroll
     for (int k = 0; k < 5; k++) v[k] = u[k] * is;
-    return sr_c2p_fast(P, v, flags);
+    return sr_c2p_fast<false>(P, v, flags);
 }
 CG_D void gr_prim_fast(const SRFastParams& P, const float* u, const GRMet& M, float* p, int* flags) {
     const SRPrim32 c = gr_c2p_fast(P, u, M, flags);
@@ -117,18 +117,21 @@ CG_D void gr_cons_fast(const SRFastParams& P, const float* p, const GRMet& M, fl
 
 // BlackHoleEuler/BlackHoleEulerStateVector.cpp:159-250 (x) and :259-350 (y): the flux of a
 // conserved state, through its primitive recovery
-template <int AXIS>
-CG_D void gr_flux_fast(const SRFastParams& P, const float* u, const GRMet& M, float* f, int* flags) {
+CG_D void gr_flux_along(int axis, const SRFastParams& P, const float* u, const GRMet& M, float* f, int* flags) {
     const SRPrim32 c = gr_c2p_fast(P, u, M, flags);
     const float as = M.al * M.sg;
     const float rhw = c.rho * c.h * c.W * c.W;
-    const float vn = AXIS == 0 ? c.vx : c.vy;
-    const float w = vn - fdiv(M.be[AXIS], M.al);
+    const float vn = axis == 0 ? c.vx : c.vy;
+    const float w = vn - fdiv(axis == 0 ? M.be[0] : M.be[1], M.al);
     f[0] = as * (c.rho * c.W * w);
-    f[1] = as * (rhw * c.vx * w + (AXIS == 0 ? c.p : 0.0f));
-    f[2] = as * (rhw * c.vy * w + (AXIS == 1 ? c.p : 0.0f));
+    f[1] = as * (rhw * c.vx * w + (axis == 0 ? c.p : 0.0f));
+    f[2] = as * (rhw * c.vy * w + (axis == 1 ? c.p : 0.0f));
     f[3] = as * (rhw * c.vz * w);
     f[4] = as * (((rhw - c.p) - c.rho * c.W) * w + c.p * vn);
+}
+template <int AXIS>
+CG_D void gr_flux_fast(const SRFastParams& P, const float* u, const GRMet& M, float* f, int* flags) {
+    gr_flux_along(AXIS, P, u, M, f, flags);
 }
 
 // Half-step evolution (Solvers/BlackHoleEulerSolvers.cpp:234-307) of the cell with primitive
@@ -235,75 +238,90 @@ CG_D void gr_source_fast(const SRFastParams& P, const float* u, const GRMet& M, 
     for (int k = 0; k < 5; k++) s[k] = f * S[k];
 }
 
-// Fractional evolution on frozen neighbours (Solvers/BlackHoleEulerSolvers.cpp:159-232): primitive
-// neighbours l | r with centres Ml, Mr (where their extrapolated fluxes are also taken), the cell's
+// Fractional evolution on frozen neighbours (Solvers/BlackHoleEulerSolvers.cpp:159-232): the neighbours'
+// conserved states ul | ur at their centres Ml, Mr (where the extrapolated fluxes are also taken), the cell's
 // primitives m; o receives the cell's primitives after frac * dt.
-template <int AXIS, int LIM>
-CG_D void gr_fraction_fast(const SRFastParams& P, const NewtonFastParams& NP, float frac, const float* l,
-                           const float* m, const float* r, const GRMet& Ml, const GRMet& Mc, const GRMet& Mr,
+template <int LIM>
+CG_D void gr_fraction_fast(int axis, const SRFastParams& P, const NewtonFastParams& NP, float frac, const float* ul,
+                           const float* m, const float* ur, const GRMet& Ml, const GRMet& Mc, const GRMet& Mr,
                            float dtdx, float* o, int* flags) {
-    float ul[5], um[5], ur[5], sl[5], a[5], b[5], Fa[5], Fb[5], nu[5];
-    gr_cons_fast(P, l, Ml, ul);
+    float um[5], sl[5], a[5], b[5], Fa[5], Fb[5], nu[5];
     gr_cons_fast(P, m, Mc, um);
-    gr_cons_fast(P, r, Mr, ur);
     nf_slope<LIM>(NP, ul, um, ur, sl);
 #pragma unroll
     for (int k = 0; k < 5; k++) { a[k] = fmaf(-0.5f, sl[k], um[k]); b[k] = fmaf(0.5f, sl[k], um[k]); }
-    gr_flux_fast<AXIS>(P, a, Ml, Fa, flags);
-    gr_flux_fast<AXIS>(P, b, Mr, Fb, flags);
+    gr_flux_along(axis, P, a, Ml, Fa, flags);
+    gr_flux_along(axis, P, b, Mr, Fb, flags);
     const float s = frac * dtdx;
 #pragma unroll
     for (int k = 0; k < 5; k++) nu[k] = fmaf(s, Fa[k] - Fb[k], um[k]);
     gr_prim_fast(P, nu, Mc, o, flags);
 }
 
+// A frozen neighbour's conserved state: from the primitives recovered from its conserved state (the
+// reference converts back and forth, Solvers/BlackHoleEulerForcingSolver.cpp:72-99).
+CG_D void gr_frozen_fast(const SRFastParams& P, const float* p, const GRMet& M, float* u, int* flags) {
+    float c[5], q[5];
+    gr_cons_fast(P, p, M, c);
+    gr_prim_fast(P, c, M, q, flags);
+    gr_cons_fast(P, q, M, u);
+}
+
 // Classical RK4 on the source with interleaved fractional sweeps
 // (Solvers/BlackHoleEulerForcingSolver.cpp:3-185; the solvers call it with bias 0 and limiter 1,
-// Solvers/BlackHoleEulerSecondOrderSolver.cpp:195-209).  cl..cb: the neighbours' and the cell's
-// conserved states at their centres (l, r along x; t, b along y); out: the cell's primitives.
+// Solvers/BlackHoleEulerSecondOrderSolver.cpp:195-209).  cm: the cell's conserved state at its centre; L, R (along
+// x), Tp, B (along y): the neighbours' at theirs, as the fractional sweeps read them (gr_frozen_fast), the same
+// for all stages; out: the cell's primitives.
 template <int LIM>
-CG_D void gr_rk_fast(const SRFastParams& P, const NewtonFastParams& NP, int dims, const float* cl, const float* cm,
-                     const float* cr, const float* ct, const float* cb, const GRMet& Ml, const GRMet& Mc,
+CG_D void gr_rk_fast(const SRFastParams& P, const NewtonFastParams& NP, int dims, const float* L, const float* cm,
+                     const float* R, const float* Tp, const float* B, const GRMet& Ml, const GRMet& Mc,
                      const GRMet& Mr, const GRMet& Mt, const GRMet& Mb, const GRSrc& X, float dt, float dtdx,
                      float* out, int* flags) {
-    float L[5], R[5], Tp[5], B[5];
-    gr_prim_fast(P, cl, Ml, L, flags);
-    gr_prim_fast(P, cr, Mr, R, flags);
-    if (dims == 2) {
-        gr_prim_fast(P, ct, Mt, Tp, flags);
-        gr_prim_fast(P, cb, Mb, B, flags);
-    }
-    float k[4][5];
-    {
-        float s[5];
-        gr_source_fast(P, cm, Mc, X, s, flags);
+    // out = cm + (k0 + 2 k1 + 2 k2 + k3) / 6; one copy of the source term for the four stages
+    float k[5], k0[5], k1[5], k2[5], c[5], nc[5];
 #pragma unroll
-        for (int i = 0; i < 5; i++) k[0][i] = dt * s[i];
-    }
+    for (int i = 0; i < 5; i++) c[i] = cm[i];
 #pragma unroll 1
-    for (int stage = 0; stage < 3; stage++) {
-        float st[5], Mp[5], E[5], c[5], s[5];
-        const float h = stage < 2 ? 0.5f : 1.0f;
-#pragma unroll
-        for (int i = 0; i < 5; i++) st[i] = fmaf(h, k[stage][i], cm[i]);
-        gr_prim_fast(P, st, Mc, Mp, flags);
-        if (dims == 1) {
-            gr_fraction_fast<0, LIM>(P, NP, stage < 2 ? 0.5f : 1.0f, L, Mp, R, Ml, Mc, Mr, dtdx, E, flags);
-        } else {
-            const float fx = stage < 2 ? 0.25f : 0.5f, fy = stage < 2 ? 0.5f : 1.0f;
-            float E1[5], E2[5];
-            gr_fraction_fast<0, LIM>(P, NP, fx, L, Mp, R, Ml, Mc, Mr, dtdx, E1, flags);
-            gr_fraction_fast<1, LIM>(P, NP, fy, Tp, E1, B, Mt, Mc, Mb, dtdx, E2, flags);
-            gr_fraction_fast<0, LIM>(P, NP, fx, L, E2, R, Ml, Mc, Mr, dtdx, E, flags);
-        }
-        gr_cons_fast(P, E, Mc, c);
+    for (int stage = 0;; stage++) {
+        float s[5];
         gr_source_fast(P, c, Mc, X, s, flags);
 #pragma unroll
-        for (int i = 0; i < 5; i++) k[stage + 1][i] = dt * s[i];
-    }
-    float nc[5];
+        for (int i = 0; i < 5; i++) {
+            k[i] = dt * s[i];
+            if (stage == 0) k0[i] = k[i];
+            else if (stage == 1) k1[i] = k[i];
+            else if (stage == 2) k2[i] = k[i];
+        }
+        if (stage == 3) break;
+        float st[5], Mp[5];
+        const float h = stage < 2 ? 0.5f : 1.0f;
 #pragma unroll
-    for (int i = 0; i < 5; i++) nc[i] = cm[i] + (1.0f / 6.0f) * (k[0][i] + 2.0f * k[1][i] + 2.0f * k[2][i] + k[3][i]);
+        for (int i = 0; i < 5; i++) st[i] = fmaf(h, k[i], cm[i]);
+        gr_prim_fast(P, st, Mc, Mp, flags);
+        // X, Y, X by one copy of the code (three made the kernel wait for instructions a quarter of the time)
+        const float fx = dims == 1 ? (stage < 2 ? 0.5f : 1.0f) : (stage < 2 ? 0.25f : 0.5f), fy = stage < 2 ? 0.5f : 1.0f;
+#pragma unroll 1
+        for (int part = 0; part < (dims == 1 ? 1 : 3); part++) {
+            const bool y = part == 1;
+            float a[5], b[5], E[5];
+            GRMet Ma = Ml, Mz = Mr;
+#pragma unroll
+            for (int i = 0; i < 5; i++) {
+                a[i] = y ? Tp[i] : L[i];
+                b[i] = y ? B[i] : R[i];
+            }
+            if (y) {
+                Ma = Mt;
+                Mz = Mb;
+            }
+            gr_fraction_fast<LIM>(y ? 1 : 0, P, NP, y ? fy : fx, a, Mp, b, Ma, Mc, Mz, dtdx, E, flags);
+#pragma unroll
+            for (int i = 0; i < 5; i++) Mp[i] = E[i];
+        }
+        gr_cons_fast(P, Mp, Mc, c);
+    }
+#pragma unroll
+    for (int i = 0; i < 5; i++) nc[i] = cm[i] + (1.0f / 6.0f) * (k0[i] + 2.0f * k1[i] + 2.0f * k2[i] + k[i]);
     gr_prim_fast(P, nc, Mc, out, flags);
 }
 
