@@ -41,18 +41,78 @@ void run_tiles(const ExactStages<Sys>& S, const SweepArgs& a) {
     }
 }
 
-// X sweeps take one-warp tiles (30 of 32 cells update) where they waste fewer threads on the row's end than
-// the larger ones (126 of 128), or where those would not give every SM a block.  389 x 509 (544 threads a
+template <class Sys, int AXIS, int NT, int LC>
+void run_pairs(const ExactStages<Sys>& S, const SweepArgs& a) {
+    constexpr int T = NT / 2 / LC - 2;
+    const Geom& G = a.G;
+    const TileArgs A = tile_args(a);
+    const dim3 grid = AXIS == 0 ? dim3((G.nx + T - 1) / T, G.ny) : dim3((G.nx + LC - 1) / LC, (G.ny + T - 1) / T);
+    if (a.out.mask) exact_pair_kernel<Sys, AXIS, NT, LC, true><<<grid, NT, 0, a.stream>>>(S, A);
+    else exact_pair_kernel<Sys, AXIS, NT, LC, false><<<grid, NT, 0, a.stream>>>(S, A);
+}
+
+// SLIC sweeps of at most five warps of cells to an SM go two threads to a cell (1000 cells in 1D: 20.4 -> 15.9 us per
+// step; 128^2 with a finer level, every launch this small: 12.5 -> 12.2 ms per run; at 9.5 warps to an SM, SR
+// 181 x 230, the pairs' extra work costs more than it hides: 340 -> 398).  Masked sweeps count the cells of the
+// whole level, of which few update, so up to twenty.
+// Otherwise X sweeps take one-warp tiles (30 of 32 cells update) where they waste fewer threads on the row's end
+// than the larger ones (126 of 128), or where those would not give every SM a block.  389 x 509 (544 threads a
 // row instead of 640): 349 -> 305 us per step; 1024^2 (1120 against 1152): 1613 -> 1532; SR 512^2 1874 -> 1690.
+// (Blocks of several lines shaped to fill whole waves, as the black hole's below, measured 303 -> 310 .. 341,
+// 1532 -> 1456 .. 1655 and 1690 -> 1602 .. 1928 for caps of 64 to 512 threads: no shape was better at all three.)
 template <class Sys>
 cudaError_t run_sweep(const Sys& sys, const SweepArgs& a) {
     const ExactStages<Sys> S{sys, make_bias(a.bias), a.lim};
     const int wide = (a.G.nx + 125) / 126;
+    const long long warps = (long long)((a.G.nx + 29) / 30) * a.G.ny;
+    if (a.order == 2 && warps <= (long long)(a.out.mask ? 20 : 5) * device_sm_count()) {
+        if (a.G.axis == 1) run_pairs<Sys, 1, 256, 4>(S, a);
+        else run_pairs<Sys, 0, 64, 1>(S, a);
+        count_launch();
+        return cudaGetLastError();
+    }
     if (a.G.axis == 1) run_tiles<Sys, 1, 128, 4>(S, a);
     else if ((a.G.nx + 29) / 30 * 32 <= wide * 128 || wide * (long long)a.G.ny < device_sm_count()) run_tiles<Sys, 0, 32, 1>(S, a);
     else run_tiles<Sys, 0, 128, 1>(S, a);
     count_launch();
     return cudaGetLastError();
+}
+
+// Black-hole sweeps of at most five warps of cells to an SM take two threads to an interface: 150^2 2196 -> 1835 us
+// per step with the launch shapes below (200^2, at 8.2 warps: 2635 without, 2730 with).
+bool gr_pairs(const Geom& G) { return (long long)G.nx * G.ny <= 5ll * 32 * device_sm_count(); }
+
+// Shape of a black-hole sweep's blocks: `lines` lines by `points` interfaces (one fewer cells update), `each`
+// threads to an interface.  Of the ways to cut a line into equal pieces and to put pieces together, the one whose
+// waves of blocks cost least: a wave has its warps' work and about ten warps' worth of latency.  A fixed 64 or
+// 128 threads left the last wave and the last tile of a line nearly empty, and blocks that run apart
+// fetch the 100 KB of code apart: 400^2 13.7 -> 8.6 ms per step, with the source step's lockstep blocks.
+struct TileShape { int points, lines, threads; size_t bytes; };
+TileShape tile_shape(int n, int lines, int each) {
+    constexpr int kWaveWarps = 10, kWarps = kLockThreads / 32;
+    TileShape best{0, 0, 0, 0};
+    long long cost = 0;
+    const long long sms = device_sm_count();
+    const int most = kLockThreads / each;
+    int m = (n + most - 2) / (most - 1);
+    for (int tried = 0; tried < 24 && m <= n; tried++, m++) {
+        const int P = (n + m - 1) / m + 1;
+        if (best.points && P < 17) break;
+        for (int lc = 1; lc * P <= most && lc <= lines; lc++) {
+            const size_t bytes = (size_t)lc * (5 * (2 * P + 3) * sizeof(double) + P + 1);
+            if (bytes > 48 * 1024) break;
+            const int warps = (P * lc * each + 31) / 32, resident = kWarps / warps;
+            const long long blocks = (long long)((n + P - 2) / (P - 1)) * ((lines + lc - 1) / lc);
+            const long long slots = sms * resident, waves = (blocks + slots - 1) / slots;
+            const long long per_sm = waves == 1 ? (blocks + sms - 1) / sms : resident;
+            const long long c = waves * (kWaveWarps + per_sm * warps);
+            if (!best.points || c < cost) {
+                best = TileShape{P, lc, warps * 32, bytes};
+                cost = c;
+            }
+        }
+    }
+    return best;
 }
 
 GRExact make_gr(const SweepArgs& a, int* status = nullptr) { return GRExact(a.gamma, a.bh, a.dx, status); }
@@ -65,8 +125,14 @@ cudaError_t launch_sweep_exact(const SweepArgs& a) {
     const GRExact S = make_gr(a, a.out.status);
     const TileArgs A = tile_args(a);
     const Geom& G = a.G;
-    if (G.axis == 0) gr_tile_kernel<0, 64, 1><<<dim3((G.nx + 62) / 63, G.ny), 64, 0, a.stream>>>(S, A);
-    else gr_tile_kernel<1, 128, 4><<<dim3((G.nx + 3) / 4, (G.ny + 30) / 31), 128, 0, a.stream>>>(S, A);
+    const bool pair = gr_pairs(G);
+    const int n = G.axis == 0 ? G.nx : G.ny, lines = G.axis == 0 ? G.ny : G.nx;
+    const TileShape h = tile_shape(n, lines, pair ? 2 : 1);
+    const int groups = (lines + h.lines - 1) / h.lines, tiles = (n + h.points - 2) / (h.points - 1);
+    const dim3 grid(G.axis == 0 ? tiles : groups, G.axis == 0 ? groups : tiles);
+    const auto kernel = G.axis == 0 ? (pair ? gr_tile_kernel<0, true> : gr_tile_kernel<0, false>)
+                                    : (pair ? gr_tile_kernel<1, true> : gr_tile_kernel<1, false>);
+    kernel<<<grid, h.threads, h.bytes, a.stream>>>(S, A, h.points, h.lines);
     count_launch();
     return cudaGetLastError();
 }
@@ -100,9 +166,9 @@ struct RkAt {
     CG_D Pt at(int dj, int di) const { return Pt{(j + dj) * dx, (i + di) * dx, 0.0}; }
 };
 struct RkCell { V5<double> c[5]; };  // primitives of the left, right, top and bottom neighbours and of the cell
-template <class T>
-CG_D V5<T> rk_source_cell(const GRExact* S, int dims, const RkCell& c, RkAt a, double dt, const StepRatio& sr,
-                          const Bias& w, int lim) {
+template <class T, class Team>
+CG_D V5<T> rk_source_cell(const Team& team, const GRExact* S, int dims, const RkCell& c, RkAt a, double dt,
+                          const StepRatio& sr, const Bias& w, int lim) {
     V5<T> u[5];
     Metric<T> g;
 #pragma unroll 1
@@ -114,24 +180,32 @@ CG_D V5<T> rk_source_cell(const GRExact* S, int dims, const RkCell& c, RkAt a, d
         gr_metric(S, a.at(n == 0 ? -1 : n == 1 ? 1 : 0, n == 2 ? -1 : n == 3 ? 1 : 0), &g);
         u[n] = gr_cons(S, &g, p);
     }
-    const V5<T> nc = rk_cell_exact(S, dims, u, a.at(0, 0), a.dx, dt, sr, w, lim, &g);
+    const V5<T> nc = rk_cell_exact(team, S, dims, u, a.at(0, 0), a.dx, dt, sr, w, lim, &g);
     return gr_prim(S, &g, nc);
 }
 __device__ __noinline__ V5<double> slow_rk(GRExact S, int dims, RkCell c, RkAt a, double dt, StepRatio sr, Bias w, int lim) {
-    return rk_source_cell<double>(&S, dims, c, a, dt, sr, w, lim);
+    return rk_source_cell<double>(OneThread{}, &S, dims, c, a, dt, sr, w, lim);
 }
 
-__global__ void __launch_bounds__(64) rk_source_kernel(const __grid_constant__ GRExact sys, Geom G, double dx, Bias w,
-                                                       int lim, const double* __restrict__ src, double* __restrict__ dst,
-                                                       DtSrc ds) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y;
-    if (j >= G.nx) return;
+// One thread per cell, 350 000 instructions a warp out of 100 KB of code: with a warp or two to a scheduler, the
+// instruction fetches bound it (a third of a warp's time).  A block has all the cells that an SM gets
+// (up to 384; whole waves of blocks), and its warps run the stages in lockstep, so that one fetch serves them:
+// without the barriers 150^2 is 2020 instead of 1820 us per step and 400^2 9585 instead of 8570.  (Two threads
+// per cell, one for each side's neighbours, have 0.7 of the instructions in a row, but twice the warps: 2000.)
+struct Lockstep { CG_D void sync() const { __syncthreads(); } };  // threads that have left do not count
+__global__ void __launch_bounds__(kLockThreads) rk_source_kernel(const __grid_constant__ GRExact sys, Geom G, double dx,
+                                                                 Bias w, int lim, const double* __restrict__ src,
+                                                                 double* __restrict__ dst, DtSrc ds) {
+    const size_t cell = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(cell / G.nx), j = (int)(cell - (size_t)i * G.nx);
     const size_t idx = (size_t)i * G.pitch + j;
     double dt;
-    if (!ds.get(dt) || gr_excised_near(sys.bh, G.dims, i, j, dx, 1)) {
+    const bool in = i < G.ny, act = in && ds.get(dt) && !gr_excised_near(sys.bh, G.dims, i, j, dx, 1);
+    if (!act) {
+        if (in) {
 #pragma unroll
-        for (int f = 0; f < 5; f++) dst[f * G.fstride + idx] = src[f * G.fstride + idx];
+            for (int f = 0; f < 5; f++) dst[f * G.fstride + idx] = src[f * G.fstride + idx];
+        }
         return;
     }
     auto ld = [&](int ii, int jj, V5<double>& p) {
@@ -149,7 +223,7 @@ __global__ void __launch_bounds__(64) rk_source_kernel(const __grid_constant__ G
     ld(i, j, c.c[4]);
     const RkAt at{j, G.dims == 1 ? 0 : i, dx};
     const StepRatio sr = ds.ratio(dt, dx);
-    const V5<xd> nc = rk_source_cell<xd>(&sys, G.dims, c, at, dt, sr, w, lim);
+    const V5<xd> nc = rk_source_cell<xd>(Lockstep{}, &sys, G.dims, c, at, dt, sr, w, lim);
     V5<double> o;
     store5(nc.v, o.v);
     if (any_nonfinite(nc.v, 5)) o = slow_rk(sys, G.dims, c, at, dt, sr, w, lim);
@@ -158,9 +232,11 @@ __global__ void __launch_bounds__(64) rk_source_kernel(const __grid_constant__ G
 }
 
 cudaError_t launch_rk_source_exact(const SweepArgs& a) {
-    dim3 grid((a.G.nx + 63) / 64, a.G.ny);
-    rk_source_kernel<<<grid, 64, 0, a.stream>>>(make_gr(a, a.out.status), a.G, a.dx, make_bias(a.bias), a.lim,
-                                                (const double*)a.src, (double*)a.dst, a.ds);
+    const long long cells = (long long)a.G.nx * a.G.ny, sms = device_sm_count();
+    const long long waves = (cells + sms * kLockThreads - 1) / (sms * kLockThreads);
+    const int threads = (int)((cells + sms * waves - 1) / (sms * waves) + 31) / 32 * 32;
+    rk_source_kernel<<<(unsigned)((cells + threads - 1) / threads), threads, 0, a.stream>>>(
+        make_gr(a, a.out.status), a.G, a.dx, make_bias(a.bias), a.lim, (const double*)a.src, (double*)a.dst, a.ds);
     count_launch();
     return cudaGetLastError();
 }
@@ -705,7 +781,7 @@ __global__ void iface_kernel(IfaceArgs A, NewtonExact nw, SRExact sr, const __gr
                 u[2].v[f] = dims == 2 ? a[15 + f] : 0.0;
                 u[3].v[f] = dims == 2 ? a[20 + f] : 0.0;
             }
-            give(rk_cell_exact(&gr, dims, u, q, A.dx, A.dt, make_ratio(A.dt, A.dx), make_bias(A.bias), A.lim, &g), o);
+            give(rk_cell_exact(OneThread{}, &gr, dims, u, q, A.dx, A.dt, make_ratio(A.dt, A.dx), make_bias(A.bias), A.lim, &g), o);
         }
     }
 }

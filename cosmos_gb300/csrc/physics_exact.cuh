@@ -845,57 +845,70 @@ CG_D void force_exact(const Sys& S, const T* L, const T* R, Pt xf, int axis, dou
 // centred at xf + dx/2, then FORCE at xf.  c: the four cells around the interface; order 1 takes the
 // two middle cells themselves.  The metric is formed once per point; the evolutions' centres are the
 // points where FORCE converts the face states.
+// One side of it: from the three cells around the left (side 0) or right (1) cell, its face state at xf,
+// conserved at the cell's centre as FORCE has it, and its flux.
 template <class T>
-CG_D void gr_interface(const GRExact* S, const V5<T>* c, int order, Pt xf, int axis, double dx, const StepRatio& st,
-                       const Bias& w, int lim, T* F) {
-    V5<T> uf[2], ff[2];  // conserved face states and their fluxes
+CG_D void gr_interface_side(const GRExact* S, const V5<T>* c, int side, int order, Pt xf, int axis, double dx,
+                            const StepRatio& st, const Bias& w, int lim, V5<T>& u, V5<T>& f) {
     Metric<T> gc;
-#pragma unroll 1
-    for (int side = 0; side < 2; side++) {
-        const Pt xc = shift_pt(xf, axis, side == 0 ? -(dx * 0.5) : dx * 0.5);
-        gr_metric(S, xc, &gc);
-        V5<T> face = c[1 + side];
-        if (order == 2) {
-            Metric<T> go;
-            const V5<T> um = gr_cons(S, &gc, c[1 + side]);
-            gr_metric(S, shift_pt(xc, axis, -dx), &go);
-            const V5<T> ul = gr_cons(S, &go, c[side]);
-            gr_metric(S, shift_pt(xc, axis, dx), &go);
-            const V5<T> ur = gr_cons(S, &go, c[2 + side]);
-            V5<T> UL, UR;
+    const Pt xc = shift_pt(xf, axis, side == 0 ? -(dx * 0.5) : dx * 0.5);
+    gr_metric(S, xc, &gc);
+    V5<T> face = c[1];
+    if (order == 2) {
+        Metric<T> go;
+        const V5<T> um = gr_cons(S, &gc, c[1]);
+        gr_metric(S, shift_pt(xc, axis, -dx), &go);
+        const V5<T> ul = gr_cons(S, &go, c[0]);
+        gr_metric(S, shift_pt(xc, axis, dx), &go);
+        const V5<T> ur = gr_cons(S, &go, c[2]);
+        V5<T> UL, UR;
 #pragma unroll
-            for (int k = 0; k < 5; k++) {
-                const T hs = half_slope(um.v[k] - ul.v[k], ur.v[k] - um.v[k], w, lim);
-                UL.v[k] = um.v[k] - hs;
-                UR.v[k] = um.v[k] + hs;
-            }
-            // the face wanted lies at xc + dx/2 (left cell) or xc - dx/2 (right cell)
-            const T s = half(T(st.d));
-            gr_metric(S, shift_pt(xc, axis, side == 0 ? -(dx * 0.5) : dx * 0.5), &go);
-            const V5<T> V = side == 0 ? UL : UR;
-            V5<T> X = side == 0 ? UR : UL;
-            const V5<T> fo = gr_flux(S, &go, V, axis);
-            gr_metric(S, shift_pt(xc, axis, side == 0 ? dx * 0.5 : -(dx * 0.5)), &go);
-            const V5<T> fi = gr_flux(S, &go, X, axis);
-#pragma unroll
-            for (int k = 0; k < 5; k++)
-                X.v[k] = X.v[k] + (s * (side == 0 ? fo.v[k] - fi.v[k] : fi.v[k] - fo.v[k]));
-            face = gr_prim(S, &go, X);
+        for (int k = 0; k < 5; k++) {
+            const T hs = half_slope(um.v[k] - ul.v[k], ur.v[k] - um.v[k], w, lim);
+            UL.v[k] = um.v[k] - hs;
+            UR.v[k] = um.v[k] + hs;
         }
-        uf[side] = gr_cons(S, &gc, face);
-        ff[side] = gr_flux(S, &gc, uf[side], axis);
+        // the face wanted lies at xc + dx/2 (left cell) or xc - dx/2 (right cell)
+        const T s = half(T(st.d));
+        gr_metric(S, shift_pt(xc, axis, side == 0 ? -(dx * 0.5) : dx * 0.5), &go);
+        const V5<T> V = side == 0 ? UL : UR;
+        V5<T> X = side == 0 ? UR : UL;
+        const V5<T> fo = gr_flux(S, &go, V, axis);
+        gr_metric(S, shift_pt(xc, axis, side == 0 ? dx * 0.5 : -(dx * 0.5)), &go);
+        const V5<T> fi = gr_flux(S, &go, X, axis);
+#pragma unroll
+        for (int k = 0; k < 5; k++)
+            X.v[k] = X.v[k] + (s * (side == 0 ? fo.v[k] - fi.v[k] : fi.v[k] - fo.v[k]));
+        face = gr_prim(S, &go, X);
     }
+    u = gr_cons(S, &gc, face);
+    f = gr_flux(S, &gc, u, axis);
+}
+// ... and FORCE of the two sides
+template <class T>
+CG_D void gr_interface_force(const GRExact* S, const V5<T>& uL, const V5<T>& uR, const V5<T>& fL, const V5<T>& fR,
+                             Pt xf, int axis, const StepRatio& st, T* F) {
+    Metric<T> g;
     V5<T> us;
     const T cc = T(st.c), d = T(st.d);
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        us.v[k] = half_mix(uf[0].v[k] + uf[1].v[k], ff[0].v[k] - ff[1].v[k], d);
-        F[k] = half_mix(ff[0].v[k] + ff[1].v[k], uf[0].v[k] - uf[1].v[k], cc);
+        us.v[k] = half_mix(uL.v[k] + uR.v[k], fL.v[k] - fR.v[k], d);
+        F[k] = half_mix(fL.v[k] + fR.v[k], uL.v[k] - uR.v[k], cc);
     }
-    gr_metric(S, xf, &gc);
-    const V5<T> fs = gr_flux(S, &gc, us, axis);
+    gr_metric(S, xf, &g);
+    const V5<T> fs = gr_flux(S, &g, us, axis);
 #pragma unroll
     for (int k = 0; k < 5; k++) F[k] = half(F[k] + fs.v[k]);
+}
+template <class T>
+CG_D void gr_interface(const GRExact* S, const V5<T>* c, int order, Pt xf, int axis, double dx, const StepRatio& st,
+                       const Bias& w, int lim, T* F) {
+    V5<T> u[2], f[2];
+#pragma unroll 1
+    for (int side = 0; side < 2; side++)
+        gr_interface_side(S, c + side, side, order, xf, axis, dx, st, w, lim, u[side], f[side]);
+    gr_interface_force(S, u[0], u[1], f[0], f[1], xf, axis, st, F);
 }
 
 // computeFORCEUpdate (Solvers/EulerFirstOrderSolver.cpp:96-101) of a black-hole cell at q.
@@ -950,14 +963,17 @@ CG_D void evolve_fraction_exact(const GRExact& S, double frac, const T* l, const
 // frozen and the spacetime is static: the neighbours' states as the fractional sweeps read them
 // (conserved again from their recovered primitives), the metrics and the source term's metric part
 // are formed once for the four stages.
-template <class T>
-CG_D V5<T> rk_cell_exact(const GRExact* S, int dims, const V5<T>* u, Pt q, double dx, double dt, const StepRatio& sr,
-                         const Bias& w, int lim, Metric<T>* gq) {
+// Team::sync() is called before the parts of a stage: threads that run in lockstep fetch the code together.
+struct OneThread { CG_D void sync() const {} };
+template <class Team, class T>
+CG_D V5<T> rk_cell_exact(const Team& team, const GRExact* S, int dims, const V5<T>* u, Pt q, double dx, double dt,
+                         const StepRatio& sr, const Bias& w, int lim, Metric<T>* gq) {
     Metric<T> gn[4];
     SourceMetric<T> sm;
     V5<T> un[4];
 #pragma unroll 1
     for (int n = 0; n < (dims == 2 ? 4 : 2); n++) {
+        team.sync();
         gr_metric(S, shift_pt(q, n >> 1, n & 1 ? dx : -dx), &gn[n]);
         un[n] = gr_cons(S, &gn[n], gr_prim(S, &gn[n], u[n]));
     }
@@ -973,11 +989,13 @@ CG_D V5<T> rk_cell_exact(const GRExact* S, int dims, const V5<T>* u, Pt q, doubl
         V5<T> p;
 #pragma unroll
         for (int i = 0; i < 5; i++) p.v[i] = cm.v[i] + (stage < 2 ? half(k.v[i]) : k.v[i]);
+        team.sync();
         p = gr_prim(S, gq, p);
         const double fx = dims == 1 ? (stage < 2 ? 0.5 : 1.0) : (stage < 2 ? 0.25 : 0.5), fy = stage < 2 ? 0.5 : 1.0;
 #pragma unroll 1
         for (int part = 0; part < (dims == 1 ? 1 : 3); part++) {
             const int y = part == 1;
+            team.sync();
             p = evolve_fraction_in(S, y ? fy : fx, un[2 * y], p, un[2 * y + 1], &gn[2 * y], gq, &gn[2 * y + 1], y, sr, w,
                                    lim);
         }

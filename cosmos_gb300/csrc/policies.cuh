@@ -102,6 +102,8 @@ struct OutOfLine {
     CG_D void flux(const xd* u, int axis, Pt, xd* f) const { give(x_flux(S, five(u), axis), f); }
 };
 
+struct FaceOf { V5<double> u; bool bad; };
+
 // The stages of a coordinate-free sweep on conserved states (Newtonian, SR).
 template <class Sys>
 struct ExactStages {
@@ -146,6 +148,50 @@ struct ExactStages {
         force_cons(OutOfLine<Sys>{sys}, a, b, Pt{0.0, 0.0, 0.0}, axis, 0.0, st, f);
         store5(f, o.v);
         if (any_nonfinite(f, 5)) o = slow_force(sys, uL, uR, axis, st);
+        return o;
+    }
+    // ---- the same stages in the pieces that two threads of a cell, or two interfaces, share
+    CG_D double half_slope_of(double dl, double dr) const { return half_slope(xd(dl), xd(dr), w, lim).v; }
+    // flux of a conserved state; not finite where the integer pipes have none (the stage that uses it then
+    // forms it again)
+    CG_D V5<double> flux(const V5<double>& u, int axis) const {
+        xd a[5], f[5];
+        V5<double> o;
+        load5(u.v, a);
+        OutOfLine<Sys>{sys}.flux(a, axis, Pt{0.0, 0.0, 0.0}, f);
+        store5(f, o.v);
+        return o;
+    }
+    // the face state that the extrapolated state V evolves to, FL and FR the fluxes of the cell's two
+    CG_D FaceOf face_of_side(const V5<double>& V, const V5<double>& FL, const V5<double>& FR, int axis,
+                             const StepRatio& st) const {
+        const Pt z{0.0, 0.0, 0.0};
+        const xd s = half(xd(st.d));
+        xd a[5], b[5];
+        FaceOf o;
+#pragma unroll
+        for (int k = 0; k < 5; k++) a[k] = xd(V.v[k]) + (s * (xd(FL.v[k]) - xd(FR.v[k])));
+        OutOfLine<Sys>{sys}.prim(a, z, b);
+        OutOfLine<Sys>{sys}.cons(b, z, a);
+        store5(a, o.u.v);
+        o.bad = any_nonfinite(a, 5);
+        return o;
+    }
+    // FORCE of two conserved states whose fluxes are at hand
+    CG_D V5<double> force_of(const V5<double>& uL, const V5<double>& uR, const V5<double>& fL, const V5<double>& fR,
+                             int axis, const StepRatio& st) const {
+        xd us[5], F[5], fs[5];
+        V5<double> o;
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            us[k] = half_mix(xd(uL.v[k] + uR.v[k]), xd(fL.v[k] - fR.v[k]), xd(st.d));
+            F[k] = half_mix(xd(fL.v[k] + fR.v[k]), xd(uL.v[k] - uR.v[k]), xd(st.c));
+        }
+        OutOfLine<Sys>{sys}.flux(us, axis, Pt{0.0, 0.0, 0.0}, fs);
+#pragma unroll
+        for (int k = 0; k < 5; k++) F[k] = half(F[k] + fs[k]);
+        store5(F, o.v);
+        if (any_nonfinite(F, 5)) o = slow_force(sys, uL, uR, axis, st);
         return o;
     }
     // computeFORCEUpdate, Solvers/EulerFirstOrderSolver.cpp:96-101, then setConservedVariableVector
