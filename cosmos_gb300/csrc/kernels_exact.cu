@@ -1,5 +1,7 @@
 // FP64 reference-exact kernels.  Compiled with --fmad=false so that every double operation is
 // rounded exactly as the reference's (built with -ffp-contract=off) -- results are bit-identical.
+#include <cstring>
+
 #include "exact_tiles.cuh"
 #include "launch.h"
 #include "policies.cuh"
@@ -310,10 +312,37 @@ struct ConsLoader {
                                   : ((const double*)state)[f * G.fstride + k];
         cons_of(p, q, u);
     }
+    // Newtonian and SR conversions on the integer pipes, as in the sweeps
     CG_D void cons_of(const double* p, Pt q, double* u) const {
-        if (system == 0) nw.cons(p, q, u);
-        else if (system == 1) sr.cons(p, q, u);
+        if (system == 0) give(ExactStages<NewtonExact>{nw, Bias{}, 0}.cons(five(p)), u);
+        else if (system == 1) give(ExactStages<SRExact>{sr, Bias{}, 0}.cons(five(p)), u);
         else gr.cons(p, q, u);
+    }
+    CG_D void prim_of(const double* u, Pt q, double* p) const {
+        if (system == 0) give(ExactStages<NewtonExact>{nw, Bias{}, 0}.prim(five(u)), p);
+        else if (system == 1) give(ExactStages<SRExact>{sr, Bias{}, 0}.prim(five(u)), p);
+        else gr.prim(u, q, p);
+    }
+};
+
+// Whether |x / div| >= tol, 20 times per cell of the passes below: the quotient is formed only where |x| lies
+// within 2^-50 of tol div, relatively, or that product is no ordinary number; elsewhere its rounding cannot
+// matter.  Integer comparisons of the bit patterns (a quotient on the FP64 pipe is 141 cycles a warp).
+struct Reach {
+    double div, tol;
+    long long lo, hi;  // |x| below lo: no; above hi: yes
+    Reach(double d, double t) : div(d), tol(t), lo(0), hi(0x7ff0000000000000ll) {
+        const double m = t * d;
+        if (!(d > 0.0 && t > 1e-290 && t < 1e290 && m > 1e-290 && m < 1e290)) return;
+        const double l = m * (1.0 - 0x1p-50), h = m * (1.0 + 0x1p-50);
+        memcpy(&lo, &l, sizeof lo);
+        memcpy(&hi, &h, sizeof hi);
+    }
+    CG_D bool operator()(double x) const {
+        const long long a = __double_as_longlong(x) & 0x7fffffffffffffffll;
+        if (a < lo) return false;
+        if (a > hi && a <= 0x7ff0000000000000ll) return true;
+        return fabs(x / div) >= tol;
     }
 };
 
@@ -325,8 +354,8 @@ struct ConsLoader {
 // Newtonian neighbours for every system), a threshold other than the tolerance, the coarse spacing
 // as the divisor on a finer grid (`div`) and, for the intermediate pass, `need_on` (only cells
 // whose own flag is on are tested).  dx places the cells (black-hole coordinates).
-__global__ void amr_flags_kernel(ConsLoader L, double dx, double tol, double div, int plain, int need_on,
-                                 unsigned char* coarse, unsigned char* fine) {
+__global__ void amr_flags_kernel(ConsLoader L, double dx, Reach reach, int plain, int need_on, unsigned char* coarse,
+                                 unsigned char* fine) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;
     const Geom& G = L.G;
@@ -340,7 +369,7 @@ __global__ void amr_flags_kernel(ConsLoader L, double dx, double tol, double div
         L.get(0, j + 1, Pt{(j + 1) * dx, 0.0, 0.0}, r);
 #pragma unroll
         for (int k = 0; k < 5; k++)
-            if (fabs((c[k] - l[k]) / div) >= tol || fabs((r[k] - c[k]) / div) >= tol) hit = true;
+            if (reach(c[k] - l[k]) || reach(r[k] - c[k])) hit = true;
     } else {
         L.get(i - 1, j, Pt{j * dx, (i - 1) * dx, 0.0}, t);
         L.get(i, j - 1, Pt{(j - 1) * dx, i * dx, 0.0}, l);
@@ -358,8 +387,8 @@ __global__ void amr_flags_kernel(ConsLoader L, double dx, double tol, double div
         } else L.get(i + 1, j + 1, Pt{(j + 1) * dx, (i + 1) * dx, 0.0}, b);
 #pragma unroll
         for (int k = 0; k < 5; k++)
-            if (fabs((c[k] - t[k]) / div) >= tol || fabs((b[k] - c[k]) / div) >= tol ||
-                fabs((c[k] - l[k]) / div) >= tol || fabs((r[k] - c[k]) / div) >= tol)
+            if (reach(c[k] - t[k]) || reach(b[k] - c[k]) || reach(c[k] - l[k]) ||
+                reach(r[k] - c[k]))
                 hit = true;
     }
     if (!hit) return;
@@ -395,8 +424,8 @@ cudaError_t launch_amr_flags(const SweepArgs& a, int precision, double tol, unsi
 cudaError_t launch_amr_flags_ex(const SweepArgs& a, int precision, double thr, double div, bool plain, bool need_on,
                                 unsigned char* coarse, unsigned char* fine) {
     dim3 grid((a.G.nx + 127) / 128, a.G.ny);
-    amr_flags_kernel<<<grid, 128, 0, a.stream>>>(make_loader(a, precision, a.src, a.G), a.dx, thr, div, plain ? 1 : 0,
-                                                 need_on ? 1 : 0, coarse, fine);
+    amr_flags_kernel<<<grid, 128, 0, a.stream>>>(make_loader(a, precision, a.src, a.G), a.dx, Reach(div, thr),
+                                                 plain ? 1 : 0, need_on ? 1 : 0, coarse, fine);
     count_launch();
     return cudaGetLastError();
 }
@@ -408,7 +437,7 @@ cudaError_t launch_amr_flags_ex(const SweepArgs& a, int precision, double thr, d
 // The Level-2 drivers' passes (AMR/EulerAMR.cpp:804-838 on the fine grid, :875-911 on the
 // intermediate grid) take other thresholds and the coarse spacing as divisor (`div`), and are
 // `strict`: they derefine only where every child is flagged (Level-1 tests the first child).
-__global__ void amr_derefine_kernel(ConsLoader F, Geom CG, double dx, double half, double div, int strict,
+__global__ void amr_derefine_kernel(ConsLoader F, Geom CG, double dx, Reach reach, int strict,
                                     unsigned char* coarse, unsigned char* fine, void* coarse_state) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y;
@@ -423,7 +452,7 @@ __global__ void amr_derefine_kernel(ConsLoader F, Geom CG, double dx, double hal
         F.get(0, 2 * j + 2, Pt{((j * 2) + 1) * fdx, 0.0, 0.0}, r);
 #pragma unroll
         for (int k = 0; k < 5; k++)
-            if (fabs((c[k] - l[k]) / div) >= half || fabs((r[k] - c[k]) / div) >= half) marked = true;
+            if (reach(c[k] - l[k]) || reach(r[k] - c[k])) marked = true;
         if (marked || !fine[2 * j] || (strict && !fine[2 * j + 1])) return;
         fine[2 * j] = 0;
         fine[2 * j + 1] = 0;
@@ -442,8 +471,8 @@ __global__ void amr_derefine_kernel(ConsLoader F, Geom CG, double dx, double hal
         F.get(2 * i + 2, 2 * j + 1, Pt{((j * 2) + 1) * fdx, ((i * 2) + 2) * fdx, 0.0}, b);
 #pragma unroll
         for (int k = 0; k < 5; k++)
-            if (fabs((c[k] - t[k]) / div) >= half || fabs((b[k] - c[k]) / div) >= half ||
-                fabs((c[k] - l[k]) / div) >= half || fabs((r[k] - c[k]) / div) >= half)
+            if (reach(c[k] - t[k]) || reach(b[k] - c[k]) || reach(c[k] - l[k]) ||
+                reach(r[k] - c[k]))
                 marked = true;
         const size_t fw = 2 * (size_t)CG.nx;
         if (marked || !fine[(2 * i) * fw + 2 * j]) return;
@@ -472,9 +501,7 @@ __global__ void amr_derefine_kernel(ConsLoader F, Geom CG, double dx, double hal
         for (int k = 0; k < 5; k++) s[k * CG.fstride + idx] = (float)avg[k];
     } else {
         double p[5];
-        if (F.system == 0) F.nw.prim(avg, qc, p);
-        else if (F.system == 1) F.sr.prim(avg, qc, p);
-        else F.gr.prim(avg, qc, p);
+        F.prim_of(avg, qc, p);
         double* s = (double*)coarse_state;
 #pragma unroll
         for (int k = 0; k < 5; k++) s[k * CG.fstride + idx] = p[k];
@@ -489,7 +516,7 @@ cudaError_t launch_amr_derefine_ex(const SweepArgs& a, int precision, const void
                                    double div, bool strict, unsigned char* coarse, unsigned char* fine,
                                    void* coarse_state) {
     dim3 grid((a.G.nx + 127) / 128, a.G.ny);
-    amr_derefine_kernel<<<grid, 128, 0, a.stream>>>(make_loader(a, precision, fine_state, FG), a.G, a.dx, thr, div,
+    amr_derefine_kernel<<<grid, 128, 0, a.stream>>>(make_loader(a, precision, fine_state, FG), a.G, a.dx, Reach(div, thr),
                                                     strict ? 1 : 0, coarse, fine, coarse_state);
     count_launch();
     return cudaGetLastError();
@@ -532,8 +559,7 @@ __global__ void amr_sync_kernel(ConsLoader F, Geom CG, void* coarse_state, void*
             for (int k = 0; k < 5; k++) ((float*)coarse_state)[k * CG.fstride + cidx] = (float)avg[k];
         } else {
             double p[5];
-            if (F.system == 0) F.nw.prim(avg, Pt{0.0, 0.0, 0.0}, p);
-            else F.sr.prim(avg, Pt{0.0, 0.0, 0.0}, p);
+            F.prim_of(avg, Pt{0.0, 0.0, 0.0}, p);
 #pragma unroll
             for (int k = 0; k < 5; k++) ((double*)coarse_state)[k * CG.fstride + cidx] = p[k];
         }

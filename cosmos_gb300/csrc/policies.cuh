@@ -33,6 +33,12 @@ __device__ __noinline__ V5<double> slow_cons(Sys S, V5<double> p) {
     S.cons(p.v, Pt{0.0, 0.0, 0.0}, u.v);
     return u;
 }
+template <class Sys>
+__device__ __noinline__ V5<double> slow_prim(Sys S, V5<double> u) {
+    V5<double> o;
+    S.prim(u.v, Pt{0.0, 0.0, 0.0}, o.v);
+    return o;
+}
 struct FacePair { V5<double> L, R; };
 template <class Sys>
 __device__ __noinline__ FacePair slow_faces(Sys S, V5<double> l, V5<double> m, V5<double> r, int axis, StepRatio st,
@@ -118,6 +124,15 @@ struct ExactStages {
         OutOfLine<Sys>{sys}.cons(a, Pt{0.0, 0.0, 0.0}, u);
         store5(u, o.v);
         if (any_nonfinite(u, 5)) o = slow_cons(sys, p);
+        return o;
+    }
+    CG_D V5<double> prim(const V5<double>& u) const {
+        xd a[5], p[5];
+        V5<double> o;
+        load5(u.v, a);
+        OutOfLine<Sys>{sys}.prim(a, Pt{0.0, 0.0, 0.0}, p);
+        store5(p, o.v);
+        if (any_nonfinite(p, 5)) o = slow_prim(sys, u);
         return o;
     }
     // conserved face states of the cell m after its half-step evolution (each through its primitives, as

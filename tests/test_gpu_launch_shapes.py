@@ -55,3 +55,28 @@ def test_masked_levels_above_the_pair_sizes(cg, oracle, system):
     assert (n, nf) == (wn, wnf) and ff.any()
     assert bit_equal(cp.reshape(-1), wcp) and bit_equal(fp.reshape(-1), wfp)
     check_invariants(cf, ff)
+
+
+@pytest.mark.parametrize("dims", [1, 2])
+def test_refinement_threshold_to_the_last_bit(cg, oracle, dims):
+    """Tolerances that equal a cell's gradient, one ulp to either side, and ones no gradient is compared with in the
+    short form (zero, negative, tiny, huge)."""
+    rng = np.random.default_rng(2)
+    shape = (60,) if dims == 1 else (20, 31)
+    s = cases.state(0, rng, shape)
+    s.reshape(-1, 5)[7, 0] = 1e250
+    dx = 1.0 / 37
+    rho = s.reshape(-1, shape[-1], 5)[0, :, 0]
+    tols = [0.0, -1.0, 1e-300, 1e300, np.inf]
+    for j in (20, 21, 25):
+        t = abs((rho[j] - rho[j - 1]) / dx)
+        tols += [t, np.nextafter(t, 0.0), np.nextafter(t, np.inf)]
+    g = cg.Grid(0, shape, dx, 1.4, cg.FP64, cg.BC_TRANSMISSIVE, None)
+    g.set_prim(s)
+    for tol in tols:
+        c0 = np.ones(int(np.prod(shape)), np.uint8)
+        f0 = np.zeros(c0.size * 2 ** dims, np.uint8)
+        c, f = g.amr_flags(tol, c0, f0)
+        wc, wf = oracle.amr_flags(0, s, dx, tol, 1.4, c0, f0, bh=None)
+        assert np.array_equal(c, wc) and np.array_equal(f, wf), tol
+    g.close()
