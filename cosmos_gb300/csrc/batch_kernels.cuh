@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_step_kernel(PolX polx0, PolY p
     for (int s = 0; s < nsteps; s++) {
         const int p = (step0 + s) & 1;
         // ---- A: per-grid time steps
-        for (int g = blockIdx.x * NT + threadIdx.x; g < B.ngrids; g += gridDim.x * NT) step_ctl_advance(&B.ctl[g]);
+        for (int g = blockIdx.x * NT + threadIdx.x; g < B.ngrids; g += gridDim.x * NT) step_ctl_advance<true>(&B.ctl[g]);
         if (!grid_sync(B.bar)) return;
         // ---- B, C, D
         for (int ph = 0; ph < 3; ph++) {
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_pair_kernel(NewtonFastParams P
     unsigned int* done = B.flow + 2;
     unsigned int* ready = B.flow + 2 + 3 * (size_t)n;
     // the time steps of the launch's first step, then the one barrier
-    for (int g = blockIdx.x * NT + threadIdx.x; g < n; g += gridDim.x * NT) step_ctl_advance(&B.ctl[g]);
+    for (int g = blockIdx.x * NT + threadIdx.x; g < n; g += gridDim.x * NT) step_ctl_advance<true>(&B.ctl[g]);
     if (!grid_sync(B.bar)) return;
     const int nb = B.nitems[0], nc = B.nitems[1];
     const int per_step = nb + nc + B.nitems[2];
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_pair_kernel(NewtonFastParams P
             if (last_phase && s + 1 < nsteps && fin == (unsigned)(s + 1) * (unsigned)B.gcount[3 * it.g + ph]) {
                 // every item of the grid's step is finished: its next time step
                 __threadfence();
-                step_ctl_advance(ctl);
+                step_ctl_advance<true>(ctl);
                 __threadfence();
                 atomicExch(&ready[it.g], (unsigned)(s + 1));
             }

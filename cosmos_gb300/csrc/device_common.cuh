@@ -96,7 +96,12 @@ struct StepNow {
     CG_D FastCoef full() const { return FastCoef{(float)r.d, (float)(0.5 * r.d), (float)(0.25 * r.c)}; }
     CG_D FastCoef halved() const { return FastCoef{(float)h.d, (float)(0.5 * h.d), (float)(0.25 * h.c)}; }
 };
+// COMPACT: the quotients share one copy of their code, for the batch, where few threads of a large kernel come here:
+// 256 FP32 grids 1.611 -> 1.590 ms per step (a step of 1000 cells in 1D: 15.9 -> 16.1 us, so not elsewhere).
+static __device__ __noinline__ double shared_quotient(double a, double b) { return xm::div(a, b); }
+template <bool COMPACT = false>
 CG_D StepNow step_now(const StepCtl* c) {
+    const auto over = [](double a, double b) { return COMPACT ? shared_quotient(a, b) : xm::div(a, b); };
     StepNow s;
     const double t = c->t, t_final = c->t_final, dx = c->dx;
     const int it = c->it;
@@ -109,11 +114,12 @@ CG_D StepNow step_now(const StepCtl* c) {
     } else {
         const unsigned long long m0 = c->smax[0], m1 = c->smax[1];  // both, so that no load waits for `it`
         const double smax = __longlong_as_double((long long)(it & 1 ? m1 : m0));
-        s.dt = c->cfl * quotient(dx, smax);
+        const double q = over(dx, smax);
+        s.dt = c->cfl * (xm::finite(q) ? q : dx / smax);
         if (it <= 5) s.dt = s.dt * 0.2;
         if ((t + s.dt) > t_final) s.dt = t_final - t;
     }
-    s.r = StepRatio{xm::div(s.dt, dx), xm::div(dx, s.dt)};
+    s.r = StepRatio{over(s.dt, dx), over(dx, s.dt)};
     s.h = StepRatio{0.5 * s.r.d, 2.0 * s.r.c};
     if (!xm::finite(s.r.d + s.r.c)) {
         s.r = make_ratio(s.dt, dx);
@@ -142,7 +148,8 @@ CG_D void step_enter(StepCtl* c, const StepNow& s, int clear) {
     c->it = it + 1;
 }
 // before a step's sweeps: they reduce into the other slot, emptied here
-CG_D void step_ctl_advance(StepCtl* c) { step_enter(c, step_now(c), (c->it + 1) & 1); }
+template <bool COMPACT = false>
+CG_D void step_ctl_advance(StepCtl* c) { step_enter(c, step_now<COMPACT>(c), (c->it + 1) & 1); }
 
 // Max of non-negative doubles (ordering of their bit patterns equals numeric ordering).
 // The slot only grows while a kernel reduces into it, so a block whose value does not exceed what
