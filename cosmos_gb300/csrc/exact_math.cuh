@@ -357,7 +357,9 @@ XM_HD bool clean5(const xd* a, xr* o) {
     return !bad;
 }
 template <int LO, int HI> XM_HD bool within(double) { return true; }
-template <int LO, int HI> XM_HD bool within(xr a) { return !xm::outside<LO, HI>(a.v); }
+template <int LO, int HI> XM_HD bool within(xr a) { return !xm::outside<LO, HI>(a.v); }  // or zero
+XM_HD bool nonzero(double) { return true; }
+XM_HD bool nonzero(xr a) { return !xm::zero_hi(a.v); }
 XM_HD double given(double a, bool) { return a; }
 XM_HD xd given(xr a, bool ok) { return xd(ok ? a.v : xm::double_of(0x7ff8000000000000ull)); }
 

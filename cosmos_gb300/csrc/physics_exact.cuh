@@ -210,7 +210,8 @@ struct GammaConst {
 // Bounds of the xr arithmetic, for inputs zero or in [2^-140, 2^100): E in [2^-192, 2^101] (or zero), q
 // after its floor in [2^-27, 2^203], dc in [2^-242, 2^114], ec in [2^-295, 2^115], ec^2 in [2^-590, 2^230];
 // x in [2^-60, 2^60) at every iteration (tested), so that every term of f and fp lies within 2^-800 .. 2^580;
-// the step's quotient is an `xd` one; W in [2^-60, 2^60) (tested), so rho h W^2 lies within 2^-560 .. 2^640
+// the step's quotient is an `xd` one; W in [2^-60, 2^60) (tested, and that it is not zero: an E of exactly zero,
+// tau = -D, makes it so, where the root's NaN is lost in the product), so rho h W^2 lies within 2^-560 .. 2^640
 // and the velocities within 2^-780 .. 2^660.
 // (Two states in one instruction stream were 7 % slower on the relativistic sweeps: their code does not fit
 // the instruction caches.)
@@ -249,7 +250,7 @@ __device__ __noinline__ C2P<T> con2prim_exact(V5<T> in, GammaConst k, double tol
     const R dx = dc * x;
     const R rt = root(R(1.0) + (R(k.gm4) * ((R(1.0) - dx) / (ec2 * (x * x)))));
     const R W = (half(ec) * x) * (R(1.0) + rt);
-    ok = ok & within<-60, 60>(W);
+    ok = ok & within<-60, 60>(W) & nonzero(W);
     const R h = R(1.0) / dx;
     R rho = D / W;
     const R rhw = (rho * h) * (W * W);
