@@ -360,6 +360,8 @@ template <int LO, int HI> XM_HD bool within(double) { return true; }
 template <int LO, int HI> XM_HD bool within(xr a) { return !xm::outside<LO, HI>(a.v); }  // or zero
 XM_HD bool nonzero(double) { return true; }
 XM_HD bool nonzero(xr a) { return !xm::zero_hi(a.v); }
+XM_HD bool bounded(double, bool) { return true; }  // whether a bound that only the unchecked arithmetic needs holds
+XM_HD bool bounded(xr, bool holds) { return holds; }
 XM_HD double given(double a, bool) { return a; }
 XM_HD xd given(xr a, bool ok) { return xd(ok ? a.v : xm::double_of(0x7ff8000000000000ull)); }
 

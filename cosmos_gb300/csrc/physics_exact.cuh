@@ -219,7 +219,7 @@ template <class T>
 __device__ __noinline__ C2P<T> con2prim_exact(V5<T> in, GammaConst k, double tol, int* status) {
     using R = typename Raw<T>::type;
     R u[5];
-    bool ok = clean5(in.v, u) & k.fits;
+    bool ok = clean5(in.v, u) & bounded(R(), k.fits);  // always in double
     const R D = u[0], Sx = u[1], Sy = u[2], Sz = u[3], tau = u[4];
     const R E = tau + D;
     const R q = (E * E) - (((Sx * Sx) + (Sy * Sy)) + (Sz * Sz));

@@ -1,9 +1,9 @@
 // Host build of the reference-exact primitive recovery and black-hole state functions
 // (cosmos_gb300/csrc/physics_exact.cuh) on conserved states taken as they come: physical ones, ones without a
 // root, and ones whose sums cancel to an exact zero (tau = -D: no energy; S = 0 at rest; tau = S = 0: no internal
-// energy).  The hardware form (double) has to be the reference's iteration written out below, status included;
-// wherever the integer-pipe form's (xd) results are finite they have to be the hardware form's bits.  Prints
-// what differs; exits non-zero if anything does.
+// energy).  The hardware form (double) has to be the reference's iteration written out below, status included,
+// for every gamma > 1; wherever the integer-pipe form's (xd) results are finite they have to be the hardware
+// form's bits.  Prints what differs; exits non-zero if anything does.
 #include "cuda_runtime.h"
 
 #include <cstdio>
@@ -167,8 +167,8 @@ static void black_hole(const GRExact& S) {
 
 int main(int argc, char** argv) {
     const long n = argc > 1 ? atol(argv[1]) : 20000;
-    const double gammas[] = {5.0 / 3.0, 4.0 / 3.0, 1.4, 2.0, 1.1, 3.0};
-    for (long i = 0; i < n; i++) recoveries(gammas[gen() % 6]);
+    const double gammas[] = {5.0 / 3.0, 4.0 / 3.0, 1.4, 2.0, 1.1, 3.0, 1.0 + 0x1p-52, 1e20};
+    for (long i = 0; i < n; i++) recoveries(gammas[gen() % 8]);
     const double hole[] = {0.05, 0.0, 0.5, 0.5, 0.0}, spinning[] = {0.05, 0.9, 0.5, 0.5, 0.0};
     const GRExact still(4.0 / 3.0, hole, 1.0 / 150), spun(5.0 / 3.0, spinning, 1.0 / 64);
     for (long i = 0; i < n; i++) black_hole(i & 1 ? still : spun);

@@ -40,8 +40,9 @@ def no_energy(shape, gamma):
 # two threads to a cell; the wide X tiles; one dimension
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape", [(33,), (20, 34), (160, 130)])
-@pytest.mark.parametrize("gamma", [2.0])
+@pytest.mark.parametrize("gamma", [2.0, 1.0 + 2.0 ** -52, 1e20])
 def test_sweeps_over_cells_without_energy(cosmos_lib, oracle, shape, gamma):
+    """(2.0), and gammas beyond the integer pipes' bounds, where the hardware form takes every stage."""
     import cosmos_gb300 as cg
     s = no_energy(shape, gamma)
     for axis in range(len(shape)):
