@@ -35,6 +35,7 @@ struct SRFastParams {
     // (g-2)/g, g/(g-1), in FP32 and for the FP64 stage
     float gr, c0, grg, g2g, hfac;
     double grd, k0d, grgd, g2gd;
+    float dc_gas;            // D / sqrt(q) below which a state may be a gas's (sr_c2p_fast)
 };
 
 inline void sr_fast_constants(SRFastParams& P, double g) {
@@ -49,6 +50,7 @@ inline void sr_fast_constants(SRFastParams& P, double g) {
     P.grg = (float)P.grgd;
     P.g2g = (float)P.g2gd;
     P.hfac = (float)(g / (g - 1.0));
+    P.dc_gas = g <= 2.0 ? 1.001f : 0.0f;
 }
 
 struct SRPrim32 {
@@ -136,41 +138,52 @@ CG_D SRPrim32 sr_c2p_fast(const SRFastParams& P, const float* u, int* flags) {
     // the quartic is a quadratic).  Cubic convergence: after a step below 1e-3 the iterate is at FP32
     // accuracy.  Over random physical states (p / rho 1e-8 .. 1e3, W up to 7) it ends after 1-3 steps with
     // the error of Newton's from 1, which takes 3-7 and one more to see that it has converged.
-    // A physical state has dc <= 1 (at rest D / (D + internal energy), less in motion): the others, mostly
-    // without a root, go to the reference's iteration at once.
-    float x = !inrange ? 0.0f : (REST ? frcp(P.gf - (P.gf - 1.0f) * dc) : 1.0f);
+    // Where the state is no gas's, the result is whatever the reference's iteration from 1 arrives at, so only a
+    // gas's states take this one: 0 < D and D^2 + S^2 <= E^2 (0 < dc <= 1, compared as an unsigned pattern, where a
+    // negative is large), q above its floor (below it, a density under about 1e-4, 25-36 % of the recoveries came
+    // out more than 1 % off the reference's), gamma <= 2 (above it hot gases have several roots), and a root of
+    // the energy's sign.  2048^2 Kelvin-Helmholtz: 575 us per step, 571 with dc <= 1 alone.
+    const bool gas = REST && inrange && __float_as_uint(dc) < __float_as_uint(P.dc_gas) && q > 1e-8f;
+    float x = !inrange ? 0.0f : (gas ? frcp(P.gf - (P.gf - 1.0f) * dc) : 1.0f);
     bool conv = false;
-    for (int it = 0; REST && inrange && dc < 1.001f && it < 4; it++) {
+    float y = 0.0f;
+    for (int it = 0; gas && it < 4; it++) {
         const float x2 = x * x, c4x = c4 * x, e3 = 3.0f * eta * c4x;
         const float f = c4x * x2 * (x - eta) + c2 * x2 + c1 * x + c0;
         const float fp = c1 + 2.0f * c2 * x + 4.0f * c4x * x2 - e3 * x;
         const float hf = c2 + 6.0f * c4x * x - e3;  // f'' / 2
         const float nx = x - fdiv(f * fp, fp * fp - f * hf);
-        conv = fabsf(nx - x) <= 1e-3f * fabsf(x) && nx > 0.0f;
+        y = ec * nx;
+        conv = fabsf(nx - x) <= 1e-3f * fabsf(x) && y > 0.0f;
         x = nx;
         if (conv) break;
     }
-    if (inrange && !conv) {  // as the reference iterates, from 1
-        x = 1.0f;
-        for (int it = 0; it < 40; it++) {
-            const float x2 = x * x;
-            const float f = c4 * x2 * x * (x - eta) + c2 * x2 + c1 * x + c0;
-            const float fp = c1 + 2.0f * c2 * x + 4.0f * c4 * x2 * x - 3.0f * eta * c4 * x2;
-            const float nx = x - fdiv(f, fp);
-            const bool done = fabsf(nx - x) <= 1e-6f * fabsf(x);
-            x = nx;
-            if (done) { conv = true; break; }
-        }
-    }
-    // W = (y + sqrt(y^2 + 4 gr (1 - dc x))) / 2, y = ec x.  The black-hole kernels keep the quotient's form, and
-    // below the two-reciprocal one: with the forms that have one reciprocal each their density error against FP64
-    // was 1.04e-6 instead of 8.5e-7 after five steps of 1024^2 accretion (Kelvin-Helmholtz: 2.29e-6 and 2.43e-6).
+    // The reference's W; a gas's is (y + sqrt(y^2 + 4 gr (1 - dc x))) / 2 with y = ec x > 0 (elsewhere y may be
+    // negative, or zero where the energy is: then the reference's W is no number and the result the floor state).
+    // The black-hole kernels keep the quotient's form, and below the two-reciprocal one: with the forms that have
+    // one reciprocal each their density error against FP64 was 1.04e-6 instead of 8.5e-7 after five steps of
+    // 1024^2 accretion (Kelvin-Helmholtz: 2.29e-6 and 2.43e-6).
     const auto lorentz_of = [&](float z) {
-        if (!REST) return 0.5f * ec * z * (1.0f + fsqrt(1.0f + fdiv(4.0f * gr * (1.0f - dc * z), ec * ec * z * z)));
-        const float y = ec * z;
-        return 0.5f * (y + fsqrt(fmaf(y, y, 4.0f * gr * (1.0f - dc * z))));
+        return 0.5f * ec * z * (1.0f + fsqrt(1.0f + fdiv(4.0f * gr * (1.0f - dc * z), ec * ec * z * z)));
     };
-    float W = lorentz_of(x);
+    float W;
+    if (REST && conv) {
+        W = 0.5f * (y + fsqrt(fmaf(y, y, 4.0f * gr * (1.0f - dc * x))));
+    } else {
+        if (inrange) {  // as the reference iterates, from 1
+            x = 1.0f;
+            for (int it = 0; it < 40; it++) {
+                const float x2 = x * x;
+                const float f = c4 * x2 * x * (x - eta) + c2 * x2 + c1 * x + c0;
+                const float fp = c1 + 2.0f * c2 * x + 4.0f * c4 * x2 * x - 3.0f * eta * c4 * x2;
+                const float nx = x - fdiv(f, fp);
+                const bool done = fabsf(nx - x) <= 1e-6f * fabsf(x);
+                x = nx;
+                if (done) { conv = true; break; }
+            }
+        }
+        W = lorentz_of(x);
+    }
     if (inrange && (!conv || !(W <= P.w64))) {  // also a non-finite iterate
         // from the FP32 iterate unless it ran off (then from the reference's start, 1)
         const SRStage64 r = sr_c2p_stage64(P.grd, P.k0d, P.grgd, P.g2gd, D, Sx, Sy, Sz, tau, fabsf(x) < 1e3f ? x : 1.0f);
