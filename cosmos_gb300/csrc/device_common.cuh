@@ -83,6 +83,17 @@ enum : int {
     ST_NEGATIVE = 8,        // non-positive density or pressure produced by the FP32 path
 };
 
+// Product and sum rounded each by itself, also where the compiler contracts the two into one operation (the
+// units of the FP32 kernels): the controller's time and its comparison with the final time are then the same
+// in every kernel that enters a step.
+#ifdef __CUDA_ARCH__
+CG_D double rounded_product(double a, double b) { return __dmul_rn(a, b); }
+CG_D double rounded_sum(double a, double b) { return __dadd_rn(a, b); }
+#else
+CG_HD double rounded_product(double a, double b) { return a * b; }
+CG_HD double rounded_sum(double a, double b) { return a + b; }
+#endif
+
 // The next step's dt from the last CFL reduction, Solvers/EulerSolvers.cpp:130-161: dt = CFL * (dx / s_max);
 // x0.2 while it <= 5; clamped so that t + dt does not pass t_final.  The solver loop
 // `while (t < t_final)` becomes `active`.  One thread does this between two sweeps of every step, so
@@ -115,9 +126,9 @@ CG_D StepNow step_now(const StepCtl* c) {
         const unsigned long long m0 = c->smax[0], m1 = c->smax[1];  // both, so that no load waits for `it`
         const double smax = __longlong_as_double((long long)(it & 1 ? m1 : m0));
         const double q = over(dx, smax);
-        s.dt = c->cfl * (xm::finite(q) ? q : dx / smax);
-        if (it <= 5) s.dt = s.dt * 0.2;
-        if ((t + s.dt) > t_final) s.dt = t_final - t;
+        s.dt = rounded_product(c->cfl, xm::finite(q) ? q : dx / smax);
+        if (it <= 5) s.dt = rounded_product(s.dt, 0.2);
+        if (rounded_sum(t, s.dt) > t_final) s.dt = t_final - t;
     }
     s.r = StepRatio{over(s.dt, dx), over(dx, s.dt)};
     s.h = StepRatio{0.5 * s.r.d, 2.0 * s.r.c};
@@ -144,7 +155,7 @@ CG_D void step_enter(StepCtl* c, const StepNow& s, int clear) {
     c->fc[1] = s.halved();
     c->active = 1;
     c->smax[clear] = 0ull;
-    c->t = c->t + s.dt;
+    c->t = rounded_sum(c->t, s.dt);
     c->it = it + 1;
 }
 // before a step's sweeps: they reduce into the other slot, emptied here
