@@ -158,9 +158,16 @@ CG_D void step_enter(StepCtl* c, const StepNow& s, int clear) {
     c->t = rounded_sum(c->t, s.dt);
     c->it = it + 1;
 }
-// before a step's sweeps: they reduce into the other slot, emptied here
+// Before a step's sweeps.  They reduce into the other slot, emptied here; the consumed one is emptied too, as a fused
+// step leaves it, so that the two forms may follow one another in any order (a fused step reduces into the
+// slot that the step before it consumed, and does not empty it first).
 template <bool COMPACT = false>
-CG_D void step_ctl_advance(StepCtl* c) { step_enter(c, step_now<COMPACT>(c), (c->it + 1) & 1); }
+CG_D void step_ctl_advance(StepCtl* c) {
+    const StepNow s = step_now<COMPACT>(c);
+    const int used = c->it & 1;
+    step_enter(c, s, used ^ 1);
+    if (s.active) c->smax[used] = 0ull;
+}
 
 // Max of non-negative doubles (ordering of their bit patterns equals numeric ordering).
 // The slot only grows while a kernel reduces into it, so a block whose value does not exceed what
