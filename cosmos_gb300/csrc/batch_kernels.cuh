@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_step_kernel(PolX polx0, PolY p
     for (int s = 0; s < nsteps; s++) {
         const int p = (step0 + s) & 1;
         // ---- A: per-grid time steps
-        for (int g = blockIdx.x * NT + threadIdx.x; g < B.ngrids; g += gridDim.x * NT) step_ctl_advance<true>(&B.ctl[g]);
+        for (int g = blockIdx.x * NT + threadIdx.x; g < B.ngrids; g += gridDim.x * NT) step_ctl_advance(&B.ctl[g]);
         if (!grid_sync(B.bar)) return;
         // ---- B, C, D
         for (int ph = 0; ph < 3; ph++) {
@@ -221,6 +221,28 @@ CG_D bool flow_wait(const unsigned int* c, unsigned int target, GridBarrier* b) 
     return true;
 }
 
+// The next time step of one grid of an FP32 batch: step_ctl_advance with hardware quotients and the FP32
+// coefficients alone (the same values; a batch neither logs nor prescribes time steps).  One thread of a large kernel
+// comes here once per grid and step, so what its code costs the rest of the kernel counts, not its latency: 256
+// grids 1.612 -> 1.599 ms per step against the quotients of the integer pipes.
+CG_D void batch_ctl_advance(StepCtl* c) {
+    const int it = c->it;
+    if (!(c->t < c->t_final) || it >= c->it_limit) {
+        c->active = 0;
+        c->dt = 0.0;
+        return;
+    }
+    const double dt = cfl_step(c->cfl, c->dx / __longlong_as_double((long long)c->smax[it & 1]), c->t, c->t_final, it);
+    if (!(dt > 0.0) || !isfinite(dt)) c->status |= ST_NONFINITE;
+    c->dt = dt;
+    c->fc[0] = make_fast_coef(dt, c->dx);
+    c->fc[1] = make_fast_coef(dt * 0.5, c->dx);
+    c->active = 1;
+    c->smax[0] = c->smax[1] = 0ull;
+    c->t = rounded_sum(c->t, dt);
+    c->it = it + 1;
+}
+
 // FP32 batch on cell pairs (sweep_pairs.cuh), one warp per item, no barrier after the launch's
 // first: the warps take the launch's items in order through an atomic counter (the next one is
 // taken while an item runs), and an item waits only for the items of its own grid that it reads
@@ -258,7 +280,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_pair_kernel(NewtonFastParams P
     unsigned int* done = B.flow + 2;
     unsigned int* ready = B.flow + 2 + 3 * (size_t)n;
     // the time steps of the launch's first step, then the one barrier
-    for (int g = blockIdx.x * NT + threadIdx.x; g < n; g += gridDim.x * NT) step_ctl_advance<true>(&B.ctl[g]);
+    for (int g = blockIdx.x * NT + threadIdx.x; g < n; g += gridDim.x * NT) batch_ctl_advance(&B.ctl[g]);
     if (!grid_sync(B.bar)) return;
     const int nb = B.nitems[0], nc = B.nitems[1];
     const int per_step = nb + nc + B.nitems[2];
@@ -355,7 +377,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_pair_kernel(NewtonFastParams P
             if (last_phase && s + 1 < nsteps && fin == (unsigned)(s + 1) * (unsigned)B.gcount[3 * it.g + ph]) {
                 // every item of the grid's step is finished: its next time step
                 __threadfence();
-                step_ctl_advance<true>(ctl);
+                batch_ctl_advance(ctl);
                 __threadfence();
                 atomicExch(&ready[it.g], (unsigned)(s + 1));
             }

@@ -107,12 +107,13 @@ struct StepNow {
     CG_D FastCoef full() const { return FastCoef{(float)r.d, (float)(0.5 * r.d), (float)(0.25 * r.c)}; }
     CG_D FastCoef halved() const { return FastCoef{(float)h.d, (float)(0.5 * h.d), (float)(0.25 * h.c)}; }
 };
-// COMPACT: the quotients share one copy of their code, for the batch, where few threads of a large kernel come here:
-// 256 FP32 grids 1.611 -> 1.590 ms per step (a step of 1000 cells in 1D: 15.9 -> 16.1 us, so not elsewhere).
-static __device__ __noinline__ double shared_quotient(double a, double b) { return xm::div(a, b); }
-template <bool COMPACT = false>
+// the rule itself, q = dx / s_max
+CG_D double cfl_step(double cfl, double q, double t, double t_final, int it) {
+    double dt = rounded_product(cfl, q);
+    if (it <= 5) dt = rounded_product(dt, 0.2);
+    return rounded_sum(t, dt) > t_final ? t_final - t : dt;
+}
 CG_D StepNow step_now(const StepCtl* c) {
-    const auto over = [](double a, double b) { return COMPACT ? shared_quotient(a, b) : xm::div(a, b); };
     StepNow s;
     const double t = c->t, t_final = c->t_final, dx = c->dx;
     const int it = c->it;
@@ -125,12 +126,10 @@ CG_D StepNow step_now(const StepCtl* c) {
     } else {
         const unsigned long long m0 = c->smax[0], m1 = c->smax[1];  // both, so that no load waits for `it`
         const double smax = __longlong_as_double((long long)(it & 1 ? m1 : m0));
-        const double q = over(dx, smax);
-        s.dt = rounded_product(c->cfl, xm::finite(q) ? q : dx / smax);
-        if (it <= 5) s.dt = rounded_product(s.dt, 0.2);
-        if (rounded_sum(t, s.dt) > t_final) s.dt = t_final - t;
+        const double q = xm::div(dx, smax);
+        s.dt = cfl_step(c->cfl, xm::finite(q) ? q : dx / smax, t, t_final, it);
     }
-    s.r = StepRatio{over(s.dt, dx), over(dx, s.dt)};
+    s.r = StepRatio{xm::div(s.dt, dx), xm::div(dx, s.dt)};
     s.h = StepRatio{0.5 * s.r.d, 2.0 * s.r.c};
     if (!xm::finite(s.r.d + s.r.c)) {
         s.r = make_ratio(s.dt, dx);
@@ -161,9 +160,8 @@ CG_D void step_enter(StepCtl* c, const StepNow& s, int clear) {
 // Before a step's sweeps.  They reduce into the other slot, emptied here; the consumed one is emptied too, as a fused
 // step leaves it, so that the two forms may follow one another in any order (a fused step reduces into the
 // slot that the step before it consumed, and does not empty it first).
-template <bool COMPACT = false>
 CG_D void step_ctl_advance(StepCtl* c) {
-    const StepNow s = step_now<COMPACT>(c);
+    const StepNow s = step_now(c);
     const int used = c->it & 1;
     step_enter(c, s, used ^ 1);
     if (s.active) c->smax[used] = 0ull;
