@@ -198,13 +198,19 @@ GRFastPolicy<AXIS, LIM, MASKED> make_pol(const SweepArgs& a, double bias) {
     return p;
 }
 
+bool large_grid(const Geom& G) { return (size_t)G.nx * G.ny >= (size_t)1 << 19; }
+
 constexpr int kXThreads = 64;  // 62 updates per tile; 1024^2, 6 steps: 256 threads 1389 us per step, 128 1372, 64 1363, 32 1375
 // One warp of columns per Y block, 4 rows per segment: the cells near the hole (FP64 recovery
 // stage) make some column segments several times costlier than the rest, and many small blocks
 // spread them over the SMs; a small grid has more warps too.  us per step with 4 / 8 / 16 rows: 400^2 from rest
 // 248 / 261 / 295, 60 steps 661 / 722 / 820; 1024^2 from rest 1190 / 1173 / 1228, 60 steps 1380 / 1483 / 1537.
+// With every recovery finished in FP64 the recoveries cost alike, and from 2^19 cells on the halo costs more than the
+// balance gives.  4 / 8 rows, from rest and from the states after 20 and 60 steps: 512^2 3855 / 3795, 4100 / 4112,
+// 4430 / 4464; 724^2 7300 / 7203, 7648 / 7525, 8543 / 8505; 1024^2 14063 / 13925, 14607 / 14446, 15880 / 15763;
+// 1448^2 27874 / 27576, 28770 / 28470, 30091 / 29788.
 constexpr int kYThreads = 32;
-constexpr int kYSeg = 4;
+int y_rows(const SweepArgs& a) { return a.c2p64_above > 0.0 || !large_grid(a.G) ? 4 : 8; }
 
 template <int AXIS, int LIM, bool MASKED>
 void run(const SweepArgs& a) {
@@ -218,9 +224,10 @@ void run(const SweepArgs& a) {
         if (a.order == 2) sweep_x_own_kernel<Pol, 2, kXThreads><<<grid, kXThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
         else sweep_x_own_kernel<Pol, 1, kXThreads><<<grid, kXThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out);
     } else {
-        dim3 grid((G.nx + kYThreads - 1) / kYThreads, (G.ny + kYSeg - 1) / kYSeg);
-        if (a.order == 2) sweep_y_kernel<Pol, 2, kYThreads><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out, kYSeg);
-        else sweep_y_kernel<Pol, 1, kYThreads><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out, kYSeg);
+        const int seg = y_rows(a);
+        dim3 grid((G.nx + kYThreads - 1) / kYThreads, (G.ny + seg - 1) / seg);
+        if (a.order == 2) sweep_y_kernel<Pol, 2, kYThreads><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out, seg);
+        else sweep_y_kernel<Pol, 1, kYThreads><<<grid, kYThreads, 0, a.stream>>>(pol, G, src, dst, a.ds, a.out, seg);
     }
 }
 
@@ -383,7 +390,7 @@ cudaError_t launch_sweep_gr_fast(const SweepArgs& a) {
 
 cudaError_t launch_rk_source_gr_fast(const SweepArgs& a) {
     const SRFastPolicy<0, 1, false> s = make_sr_fast<0, 1, false>(a.gamma, a.bias, a.G.nx, a.G.dims, a.c2p64_above);
-    const bool small = (size_t)a.G.nx * a.G.ny < (size_t)1 << 19;
+    const bool small = !large_grid(a.G);
     const int nt = small ? 32 : 64;
     dim3 grid((a.G.nx + nt - 1) / nt, a.G.ny);
     auto k = small ? (a.lim == 0 ? gr_rk_kernel<0, 32> : (a.lim == 1 ? gr_rk_kernel<1, 32> : gr_rk_kernel<2, 32>))
