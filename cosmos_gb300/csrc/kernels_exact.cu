@@ -56,7 +56,9 @@ void run_pairs(const ExactStages<Sys>& S, const SweepArgs& a) {
 // SLIC sweeps of at most five warps of cells to an SM go two threads to a cell (1000 cells in 1D: 20.4 -> 15.9 us per
 // step; 128^2 with a finer level, every launch this small: 12.5 -> 12.2 ms per run; at 9.5 warps to an SM, SR
 // 181 x 230, the pairs' extra work costs more than it hides: 340 -> 398).  Masked sweeps count the cells of the
-// whole level, of which few update, so up to twenty.
+// whole level, of which few update, so up to twenty: a whole Level-1 run of a blast on 128^2 (5 % of the finer level
+// refined) 2.79 ms with five, 2.76 with twenty (SR 5.74, 4.88); where the whole level is refined twenty costs what
+// it costs unmasked (3.16, 3.80; SR 7.31, 8.99).
 // Otherwise X sweeps take one-warp tiles (30 of 32 cells update) where they waste fewer threads on the row's end
 // than the larger ones (126 of 128), or where those would not give every SM a block.  389 x 509 (544 threads a
 // row instead of 640): 349 -> 305 us per step; 1024^2 (1120 against 1152): 1613 -> 1532; SR 512^2 1874 -> 1690.

@@ -65,8 +65,8 @@ bool field_map(CUtensorMap* m, const float* base, const Geom& G, unsigned box_x)
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// us per step, three sweeps against one launch (MinBee): 50x60 15.6 / 10.9, 193x257 18.3 / 10.9, 400^2 19.9 /
-// 13.9, 512^2 21.8 / 19.9, 640^2 26.4 / 27.2, 1024^2 43.1 / 54.1.
+// us per step, three sweeps against one launch (MinBee): 50x60 15.6 / 9.5, 193x257 18.6 / 9.7, 400^2 19.9 /
+// 12.2, 512^2 22.0 / 18.5, 547^2 24.4 / 20.0, 640^2 26.1 / 24.8, 1024^2 43.6 / 51.6.
 constexpr size_t kFusedStepCells = 300000;
 
 namespace {

@@ -200,11 +200,13 @@ GRFastPolicy<AXIS, LIM, MASKED> make_pol(const SweepArgs& a, double bias) {
 
 bool large_grid(const Geom& G) { return (size_t)G.nx * G.ny >= (size_t)1 << 19; }
 
-constexpr int kXThreads = 64;  // 62 updates per tile; 1024^2, 6 steps: 256 threads 1389 us per step, 128 1372, 64 1363, 32 1375
+// 62 updates per X tile.  us per step of 64 / 128 / 256 threads, 6 steps from rest: 200^2 101.7 / 101.5 / 103.7, 400^2
+// 223 / 226 / 226, 640^2 514 / 520 / 519, 800^2 779 / 786 / 797, 1024^2 1253 / 1260 / 1277.
+constexpr int kXThreads = 64;
 // One warp of columns per Y block, 4 rows per segment: the cells near the hole (FP64 recovery
 // stage) make some column segments several times costlier than the rest, and many small blocks
-// spread them over the SMs; a small grid has more warps too.  us per step with 4 / 8 / 16 rows: 400^2 from rest
-// 248 / 261 / 295, 60 steps 661 / 722 / 820; 1024^2 from rest 1190 / 1173 / 1228, 60 steps 1380 / 1483 / 1537.
+// spread them over the SMs; a small grid has more warps too.  us per step with 4 / 8 rows, from rest and from the
+// state after 60 steps: 400^2 216 / 231, 964 / 1079; 1024^2 1234 / 1213, 1821 / 1890.
 // With every recovery finished in FP64 the recoveries cost alike, and from 2^19 cells on the halo costs more than the
 // balance gives.  4 / 8 rows, from rest and from the states after 20 and 60 steps: 512^2 3855 / 3795, 4100 / 4112,
 // 4430 / 4464; 724^2 7300 / 7203, 7648 / 7525, 8543 / 8505; 1024^2 14063 / 13925, 14607 / 14446, 15880 / 15763;
@@ -244,8 +246,9 @@ void run_lim(const SweepArgs& a) {
 // place), so the three fractional sweeps of a stage and the four stages' source terms share one copy of the code
 // each, and the neighbours' conserved states are formed once: 1024^2 steps 1363 -> 1211 us (6 steps from rest),
 // 1760 -> 1507 (60 steps).  Sharing the neighbours' recoveries too measured 1241 us.  384 threads per SM (168
-// registers): 256 1400 us, 512 1410.  Blocks of 64 threads, of 32 on small grids (400^2: 128 threads 261 us per
-// step, 64 251, 32 228; 1024^2: 1173, 1177, 1187).
+// registers): 256 1400 us, 512 1410.  Blocks of 64 threads, of 32 below 2^19 cells: 32 / 64 / 128
+// threads, us per step of 6 from rest: 200^2 101.7 / 101.4 / 101.4, 400^2 224 / 250 / 259, 512^2 342 / 339 / 339, 640^2 514 / 513 /
+// 509, 724^2 652 / 659 / 658, 800^2 779 / 798 / 835, 1024^2 1252 / 1243 / 1237.
 template <int LIM, int NT>
 __global__ void __launch_bounds__(NT, 384 / NT) gr_rk_kernel(SRFastParams P, NewtonFastParams NP, GRTables T, Geom G, double dx,
                                                     const float* __restrict__ src, float* __restrict__ dst, DtSrc ds,

@@ -2,7 +2,7 @@
 // (small 2D grids).
 //
 // What bounds a step there is not its work but four launches in a row, each a few microseconds of start, one
-// dependent pass and a drain: 193 x 257 took 20 us per step (dt kernel 3.7, X 5.6, Y 9.3, X 6.7 under the
+// dependent pass and a drain: 193 x 257 took 18.6 us per step (dt kernel 3.7, X 5.6, Y 9.3, X 6.7 under the
 // profiler) where its memory traffic is under one.  Here a block of 16 warps takes a tile of 56 x 12 cells with
 // its halo (4 columns and 2 rows on each side) through the three sweeps in shared memory: warp w sweeps row
 // w - 2 in X, owns row w - 1 in Y (its evolution, and the flux above it) and sweeps row w in X again.  The
@@ -10,7 +10,7 @@
 // results are theirs bit for bit; the price is the halo's repeated work, 1.33 x in the rows, which is why large
 // grids keep the three sweeps.
 //
-// us per step, three sweeps against one launch: 50 x 60 15.6 -> 9.6, 193 x 257 18.3 -> 9.8, 400^2 19.9 -> 12.7.
+// The times of both forms stand at kFusedStepCells (kernels_fast.cu): 193 x 257 18.6 -> 9.7 us per step.
 // (Programmatic dependent launch of the next step's blocks measured no faster.)
 //
 // The time step: every block forms it itself (one thread, while the others load the tile) from the controller,
