@@ -111,6 +111,33 @@ static __device__ __noinline__ SRStage64 sr_c2p_stage64(double grd, double k0, d
     return SRStage64{(float)xd, false};
 }
 
+// The reference's Lorentz factor of a root z.
+CG_D float sr_lorentz(float gr, float dc, float ec, float z) {
+    return 0.5f * ec * z * (1.0f + fsqrt(1.0f + fdiv(4.0f * gr * (1.0f - dc * z), ec * ec * z * z)));
+}
+// The reference's iteration in FP32, from 1, and its Lorentz factor: out of line, for the sweeps, whose states come
+// here rarely.  Inlined at every recovery it made them wait for code (Kelvin-Helmholtz 2048^2 576 us per step, with
+// this copy 540; 120 x 150 39.7, 35.6).  The coefficients are formed again from dc and ec, so that the callers need not
+// keep them.
+struct SRRoot32 {
+    float x, W;
+    bool conv;
+};
+static __device__ __noinline__ SRRoot32 sr_c2p_reference(float gr, float c0, float grg, float g2g, float dc, float ec) {
+    const float c1 = -2.0f * dc * grg, c2 = g2g * (ec * ec - 1.0f) + 1.0f - dc * dc * gr * gr, c4 = ec * ec - 1.0f;
+    const float eta = 2.0f * dc * gr;
+    SRRoot32 r{1.0f, 0.0f, false};
+    for (int it = 0; it < 40 && !r.conv; it++) {
+        const float x = r.x, x2 = x * x;
+        const float f = c4 * x2 * x * (x - eta) + c2 * x2 + c1 * x + c0;
+        const float fp = c1 + 2.0f * c2 * x + 4.0f * c4 * x2 * x - 3.0f * eta * c4 * x2;
+        r.x = x - fdiv(f, fp);
+        r.conv = fabsf(r.x - x) <= 1e-6f * fabsf(x);
+    }
+    r.W = sr_lorentz(gr, dc, ec, r.x);
+    return r;
+}
+
 // Primitive recovery of one FP32 conserved state; sets bit 0 of *flags when neither stage converged.
 // Near the horizon the reference's recovery meets states without a physical root, whose garbage
 // primitives grow through the W cap and the fluxes to magnitudes beyond FP32's range (|S| ~ 1e30;
@@ -142,7 +169,7 @@ CG_D SRPrim32 sr_c2p_fast(const SRFastParams& P, const float* u, int* flags) {
     // gas's states take this one: 0 < D and D^2 + S^2 <= E^2 (0 < dc <= 1, compared as an unsigned pattern, where a
     // negative is large), q above its floor (below it, a density under about 1e-4, 25-36 % of the recoveries came
     // out more than 1 % off the reference's), gamma <= 2 (above it hot gases have several roots), and a root of
-    // the energy's sign.  2048^2 Kelvin-Helmholtz: 575 us per step, 571 with dc <= 1 alone.
+    // the energy's sign.
     const bool gas = REST && inrange && __float_as_uint(dc) < __float_as_uint(P.dc_gas) && q > 1e-8f;
     float x = !inrange ? 0.0f : (gas ? frcp(P.gf - (P.gf - 1.0f) * dc) : 1.0f);
     bool conv = false;
@@ -163,33 +190,33 @@ CG_D SRPrim32 sr_c2p_fast(const SRFastParams& P, const float* u, int* flags) {
     // The black-hole kernels keep the quotient's form, and below the two-reciprocal one: with the forms that have
     // one reciprocal each their density error against FP64 was 1.04e-6 instead of 8.5e-7 after five steps of
     // 1024^2 accretion (Kelvin-Helmholtz: 2.29e-6 and 2.43e-6).
-    const auto lorentz_of = [&](float z) {
-        return 0.5f * ec * z * (1.0f + fsqrt(1.0f + fdiv(4.0f * gr * (1.0f - dc * z), ec * ec * z * z)));
-    };
     float W;
     if (REST && conv) {
         W = 0.5f * (y + fsqrt(fmaf(y, y, 4.0f * gr * (1.0f - dc * x))));
+    } else if (REST && inrange) {
+        const SRRoot32 r = sr_c2p_reference(gr, c0, P.grg, P.g2g, dc, ec);
+        conv = r.conv;
+        x = r.x;
+        W = r.W;
     } else {
-        if (inrange) {  // as the reference iterates, from 1
-            x = 1.0f;
-            for (int it = 0; it < 40; it++) {
-                const float x2 = x * x;
-                const float f = c4 * x2 * x * (x - eta) + c2 * x2 + c1 * x + c0;
-                const float fp = c1 + 2.0f * c2 * x + 4.0f * c4 * x2 * x - 3.0f * eta * c4 * x2;
-                const float nx = x - fdiv(f, fp);
-                const bool done = fabsf(nx - x) <= 1e-6f * fabsf(x);
-                x = nx;
-                if (done) { conv = true; break; }
-            }
+        // the same iteration inline (as a function shared with the other the black-hole steps were 1 % slower)
+        for (int it = 0; inrange && it < 40; it++) {
+            const float x2 = x * x;
+            const float f = c4 * x2 * x * (x - eta) + c2 * x2 + c1 * x + c0;
+            const float fp = c1 + 2.0f * c2 * x + 4.0f * c4 * x2 * x - 3.0f * eta * c4 * x2;
+            const float nx = x - fdiv(f, fp);
+            const bool done = fabsf(nx - x) <= 1e-6f * fabsf(x);
+            x = nx;
+            if (done) { conv = true; break; }
         }
-        W = lorentz_of(x);
+        W = sr_lorentz(gr, dc, ec, x);
     }
     if (inrange && (!conv || !(W <= P.w64))) {  // also a non-finite iterate
         // from the FP32 iterate unless it ran off (then from the reference's start, 1)
         const SRStage64 r = sr_c2p_stage64(P.grd, P.k0d, P.grgd, P.g2gd, D, Sx, Sy, Sz, tau, fabsf(x) < 1e3f ? x : 1.0f);
         conv = r.conv;
         x = r.x;
-        W = lorentz_of(x);
+        W = sr_lorentz(gr, dc, ec, x);
     }
     SRPrim32 r;
     r.W = W;
