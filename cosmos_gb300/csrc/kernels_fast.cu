@@ -67,6 +67,10 @@ bool field_map(CUtensorMap* m, const float* base, const Geom& G, unsigned box_x)
 
 // us per step, three sweeps against one launch (MinBee): 50x60 15.6 / 9.5, 193x257 18.6 / 9.7, 400^2 19.9 /
 // 12.2, 512^2 22.0 / 18.5, 547^2 24.4 / 20.0, 640^2 26.1 / 24.8, 1024^2 43.6 / 51.6.
+// Ragged grids leave tiles nearly empty, so the tiles count too: four to an SM are two waves of resident blocks
+// (rows x columns, tiles: 25x11000, 591 21.0 / 20.7; 2600x113, 651 24.3 / 25.1; 13x20000, 716 21.3 / 24.6; 5200x57, 868
+// 25.7 / 30.5).  Six where one column of tiles holds the grid, whose sweeps leave their warps as empty (8000x8, 667
+// 27.6 / 25.9; 12000x8, 1000 35.1 / 35.2; 14900x20, 1242 41.3 / 42.4; 30000x8, 2500 68.9 / 77.3).
 constexpr size_t kFusedStepCells = 300000;
 
 namespace {
@@ -215,9 +219,11 @@ cudaError_t launch_prim_out_fast(const void* soa, double* aos, const Geom& G, in
     return cudaGetLastError();
 }
 
-// Whole steps in one launch: two-dimensional SLIC without a mask, up to kFusedStepCells cells.
+// Whole steps in one launch: two-dimensional SLIC without a mask, up to kFusedStepCells cells in a few tiles per SM.
 bool fused_step_fast(const Geom& G, int system, int order) {
-    return system == 0 && order == 2 && G.dims == 2 && G.nx >= 8 && G.ny >= 8 && (size_t)G.nx * G.ny <= kFusedStepCells;
+    if (system != 0 || order != 2 || G.dims != 2 || G.nx < 8 || G.ny < 8 || (size_t)G.nx * G.ny > kFusedStepCells) return false;
+    const long long across = (G.nx + kTileCols - 1) / kTileCols, down = (G.ny + kTileRows - 1) / kTileRows;
+    return across * down <= (across == 1 ? 6ll : 4ll) * device_sm_count();
 }
 
 namespace {

@@ -81,9 +81,10 @@ def test_four_quadrant_error(cg, oracle):
 
 
 @pytest.mark.parametrize("lim", [0, 1, 2])
-@pytest.mark.parametrize("shape", [(547, 548), (548, 548), (8, 37501)])
+@pytest.mark.parametrize("shape", [(547, 548), (548, 548), (8, 37501), (3648, 57), (3649, 57), (10944, 8), (10945, 8)])
 def test_run_equals_single_sweeps_on_both_sides(cg, shape, lim):
-    """299 756 cells (fused steps), 300 304 and 300 008 (three sweeps): the run's steps are the single sweeps'."""
+    """299 756 cells (fused steps), 300 304 and 300 008 (three sweeps); fused steps of four and six tiles per SM, and
+    a row more: the run's steps are the single sweeps'."""
     s = cases.riemann(shape, 3 + lim)
     s[..., 0] += 0.4
     s[..., 4] += 0.3
