@@ -7,8 +7,8 @@ namespace cg {
 
 namespace {
 
-// us per step of Kelvin-Helmholtz by X tile of 64 / 128 / 256 threads: 200^2 38.8 / 38.1 / 39.1, 512^2 61.4 / 62.1 / 69.4,
-// 1000^2 153.9 / 146.0 / 151.3, 1024^2 154.8 / 156.5 / 169.8, 2048^2 586.6 / 577.1 / 621.3 (256: a row's ninth tile
+// us per step of Kelvin-Helmholtz by X tile of 64 / 128 / 256 threads: 200^2 35.6 / 35.0 / 35.7, 512^2 56.8 / 58.1 / 64.7,
+// 1000^2 144.8 / 137.8 / 143.1, 1024^2 146.1 / 147.5 / 160.3, 2048^2 547.6 / 538.3 / 581.4 (256: a row's ninth tile
 // holds 16 cells); 32 threads are slower throughout (2048^2 by 8 %).
 constexpr int kXThreads = 128;
 // One-warp Y blocks whose rows fill whole waves: 128-thread blocks of 32 rows were 1.68 waves at 2048^2 (643 ->
